@@ -60,7 +60,8 @@ def parse(argv=None):
     ap.add_argument("--cong", type=int, default=512)
     ap.add_argument("--precision", default="i8",
                     choices=["fp32", "3xtf32", "tf32", "bf16", "simt", "i8"],
-                    help="DCT GEMMs: fp32 (= simt, CUDA cores), 3xtf32, tf32, bf16 (tensor cores)")
+                    help="DCT solve: fp32 (= simt = i8: fast transforms, FP64 arithmetic), 3xtf32, tf32, "
+                         "bf16 (tensor-core GEMMs)")
     ap.add_argument("--seed", type=int, default=42)
     ap.add_argument("--bh-walk", default="fast", choices=["fast", "exact"],
                     help="Barnes-Hut walk: hardware rsqrt (default) or the bit-reproducible one")
@@ -89,12 +90,11 @@ def parse(argv=None):
 
 
 PREC = {"fp32": 3, "simt": 3, "3xtf32": 0, "tf32": 1, "bf16": 2, "i8": 4}
-PREC_DTYPE = {"fp32": "f32 (DCT GEMMs FP32 on CUDA cores)",
+PREC_DTYPE = {"fp32": "f32 (fast DCT, FP64 arithmetic)",
               "3xtf32": "f32 (DCT GEMMs 3xTF32, FP32 accumulate)",
               "tf32": "f32 (DCT GEMMs TF32, FP32 accumulate)",
-              "bf16": "f32 (DCT GEMMs BF16, FP32 accumulate)", "simt": "f32",
-              "i8": "f32 (DCT GEMMs on the tensor cores from exact 8-bit slices, int32 "
-                    "accumulate)"}
+              "bf16": "f32 (DCT GEMMs BF16, FP32 accumulate)", "simt": "f32 (fast DCT, FP64 arithmetic)",
+              "i8": "f32 (fast DCT, FP64 arithmetic)"}
 
 
 # ---------------------------------------------------------------------------
@@ -547,27 +547,26 @@ def run_fluxion(args, rank, world, local_rank):
         roof["traffic"] = None  # the captures are of the default workload
     dens_roof = None
     if "density" in per_iter:
-        fl = f_alg["density"] * 6 / 4  # six GEMMs per step (no potential)
-        d_tf = fl / (per_iter["density"] * 1e-3) / 1e12
         code = PREC[args.precision]
-        halves = code != 0 and args.bins % 256 == 0  # the even/odd half products
-        executed = d_tf / 2 if halves else d_tf
-        if code == 3:
-            pk, ps = 148 * 128 * 2 * 1.965e9 / 1e12, "nominal FP32 CUDA cores 148 x 128 x 2 x 1.965 GHz"
-            bound, unit = "fp32-pipe", "TFLOP/s"
-        elif code == 4:
-            # 21 slice-pair int8 products per GEMM; int8 dense = twice the bf16 rate
-            executed *= 21
-            pk, ps = 2 * bf16, f"{src} bf16 dense x 2 (int8)"
-            bound, unit = "tensor (int8)", "TOPS"
+        if code in (3, 4):
+            # 5/2 G complex FFTs of G points (two rows each): 5 N log2 N flops
+            g = args.bins
+            fl = 2.5 * g * 5 * g * float(np.log2(g))
+            executed = fl / (per_iter["density"] * 1e-3) / 1e12
+            pk, ps = 148 * 64 * 2 * 1.965e9 / 1e12, "nominal FP64 148 x 64 x 2 x 1.965 GHz"
+            bound, unit, flops = "fp64-pipe", "TFLOP/s", "2.5 G complex FFTs of G points"
+            halves = False
         else:
+            halves = code != 0 and args.bins % 256 == 0  # the even/odd half products
+            fl = f_alg["density"] * 6 / 4  # six GEMMs per step (no potential)
+            executed = fl / (per_iter["density"] * 1e-3) / 1e12 / (2 if halves else 1)
             pk = bf16 if args.precision == "bf16" else bf16 / 2
             ps = f"{src} bf16 dense" + ("" if args.precision == "bf16" else " / 2 (tf32)")
             bound, unit = "tensor", "TFLOP/s"
-        dens_roof = {"bound": bound, "algorithmic_tflops": d_tf, "executed": executed,
+            flops = "algorithmic: the dense GEMM form, 6 x 2 G^3 per step"
+        dens_roof = {"bound": bound, "executed": executed,
                      "unit_executed": unit, "peak": pk, "frac": executed / pk,
-                     "peak_source": ps,
-                     "flops": "algorithmic: the dense GEMM form, 6 x 2 G^3 per step",
+                     "peak_source": ps, "flops": flops,
                      "note": ("split in two half-size products by the DCT's even/odd symmetry; "
                               if halves else "") + "side stream, overlapped with Barnes-Hut: its "
                                                    "span includes time it yields"}
@@ -987,11 +986,11 @@ HPWL_ITERS = (3, 10, 50)
 def run_precision(args, rank, world, local_rank):
     """The density step's precision sweep on a 4M-gate netlist from the same
     generator (die 2400 x 2400): for G = 2048 and 4096 and each DCT precision
-    (BF16, TF32, 3xTF32, SIMT FP32; FP32 accumulation throughout), the
+    (BF16, TF32, 3xTF32 GEMMs, FP32 accumulation; FP32 by fast transforms), the
     field / force / potential relative L2 error against the FP64 FFT oracle
     (scipy dctn/idctn of force_electrostatic.py), the density stage's device
-    time and GEMM throughput, and the HPWL of a plain run against the SIMT
-    FP32 run after each count of HPWL_ITERS. HPWL and energy are FP64
+    time and GEMM throughput, and the HPWL of a plain run against the FP32
+    run after each count of HPWL_ITERS. HPWL and energy are FP64
     reductions on the device."""
     if rank != 0:
         return
@@ -1006,7 +1005,7 @@ def run_precision(args, rank, world, local_rank):
     d.set_positions(p.gate_x, p.gate_y)
     area = (c.gate_widths * c.gate_heights).astype(np.float64)
     codes = {"bf16": fx.FX_DCT_BF16, "tf32": fx.FX_DCT_TF32, "3xtf32": fx.FX_DCT_FP32,
-             "i8_slices": fx.FX_DCT_I8, "fp32_simt": fx.FX_DCT_SIMT}
+             "fp32": fx.FX_DCT_I8}
     _, bf16_peak, src = peaks()
 
     def rel(a, b):
@@ -1031,11 +1030,11 @@ def run_precision(args, rank, world, local_rank):
             ctx.set_profiling(False)
             ms = ctx.stage_times()["density"][0] / reps
             # executed: the even/odd half GEMMs (G a multiple of 256, not
-            # 3xTF32) do G^3 each instead of 2 G^3; 3xTF32 runs three MMAs
-            # (FX_DCT_I8: 21 8-bit slice-pair products per GEMM, int8 ops)
+            # 3xTF32) do G^3 each instead of 2 G^3; 3xTF32 runs three MMAs.
+            # The FP32-accurate setting runs no MMAs (fast transforms).
             halves = G % 256 == 0 and code != fx.FX_DCT_FP32
-            flops = 6 * (1.0 if halves else 2.0) * G ** 3 * (
-                3 if code == fx.FX_DCT_FP32 else 21 if code == fx.FX_DCT_I8 else 1)
+            tensor = code != fx.FX_DCT_I8
+            flops = 6 * (1.0 if halves else 2.0) * G ** 3 * (3 if code == fx.FX_DCT_FP32 else 1)
             fld = float(np.sqrt((np.linalg.norm(out["ex"] - ref["ex"]) ** 2 +
                                  np.linalg.norm(out["ey"] - ref["ey"]) ** 2) /
                                 (np.linalg.norm(ref["ex"]) ** 2 + np.linalg.norm(ref["ey"]) ** 2)))
@@ -1054,22 +1053,20 @@ def run_precision(args, rank, world, local_rank):
             hp[name] = hpwl_at
             print(f"precision sweep: G={G} {name}: {time.perf_counter() - t_phase:.1f} s",
                   file=sys.stderr, flush=True)
-            # int8 dense: twice the bf16 rate (nominal ratio); tf32: half
-            peak = (bf16_peak if code == fx.FX_DCT_BF16 else
-                    2 * bf16_peak if code == fx.FX_DCT_I8 else bf16_peak / 2)
+            peak = bf16_peak if code == fx.FX_DCT_BF16 else bf16_peak / 2  # tf32: half
             rows.append({"G": G, "precision": name, "field_rel_l2": fld, "force_rel_l2": frc,
                          "phi_rel_l2": rel(out["phi"], ref["phi"]),
                          "energy_rel": abs(out["energy"] - ref["energy"]) / abs(ref["energy"]),
                          "density_ms": ms,
                          "tensor_tflops_executed": (flops / (ms * 1e-3) / 1e12
-                                                    if code != fx.FX_DCT_SIMT else None),
+                                                    if tensor else None),
                          "tensor_frac_of_measured": (flops / (ms * 1e-3) / 1e12 / peak
-                                                     if code != fx.FX_DCT_SIMT else None),
+                                                     if tensor else None),
                          "hpwl_after_iters": {str(k): v for k, v in hpwl_at.items()}})
         for r in rows:
             if r["G"] == G:
                 r["hpwl_delta_vs_fp32"] = {
-                    str(it): (hp[r["precision"]][it] - hp["fp32_simt"][it]) / hp["fp32_simt"][it]
+                    str(it): (hp[r["precision"]][it] - hp["fp32"][it]) / hp["fp32"][it]
                     for it in HPWL_ITERS}
     d.close()
     ctx.close()

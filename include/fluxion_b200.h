@@ -79,7 +79,7 @@ int fx_ctx_synchronize(fx_ctx *ctx);
 #define FX_STAGE_BH_SORT           2 /* row B: radix sort                     */
 #define FX_STAGE_BH_TREE           3 /* row B: radix tree + mass sums         */
 #define FX_STAGE_BH_WALK           4 /* row B: warp-cooperative walk          */
-#define FX_STAGE_DENSITY           5 /* row C: scatter + DCT GEMMs + field    */
+#define FX_STAGE_DENSITY           5 /* row C: scatter + DCT solve + field    */
 #define FX_STAGE_CONGESTION        6 /* rows D+F: bbox, counting, HPWL        */
 #define FX_STAGE_LEAF              7 /* row H: batched leaf placer            */
 #define FX_STAGE_FIEDLER           8 /* row G: power iteration                */
@@ -256,12 +256,9 @@ typedef struct fx_iter_cfg {
                        /* FP32 inputs, not FP32 accuracy                     */
 #define FX_DCT_TF32  1 /* single-pass TF32 inputs, FP32 accumulate           */
 #define FX_DCT_BF16  2 /* BF16 inputs, FP32 accumulate                       */
-#define FX_DCT_SIMT  3 /* FP32 CUDA-core GEMM (no tensor cores)              */
-#define FX_DCT_I8    4 /* tensor cores, FP32-accurate: each operand row split */
-                       /* into six exact 8-bit slices under a power-of-two    */
-                       /* scale, slice products accumulated exactly in int32  */
-                       /* (tcgen05 kind::i8), classes combined in FP64: the   */
-                       /* iteration's default                                  */
+#define FX_DCT_SIMT  3 /* FP32-accurate: fast transforms in FP64 arithmetic,  */
+                       /* f32 grids (within 1e-6 of FP64 at every G)          */
+#define FX_DCT_I8    4 /* the same solve (the iteration's default)             */
 
 typedef struct fx_iter_stats {
   double hpwl;            /* FP64 HPWL after the last iteration              */
@@ -473,8 +470,7 @@ typedef struct fx_job_desc {
   const fx_leaf_cfg *leaf;  /* leaf default with FX_LEAF_FAST; ECO: the iteration  */
   const fx_refine_cfg *refine; /* default with a G x G density grid, G the         */
   const fx_iter_cfg *iter;  /* multiple of 128 nearest sqrt(n) in [128, 1024],     */
-                            /* FX_DCT_SIMT below G = 1024, and a 256 x 256         */
-                            /* congestion grid)                                    */
+                            /* and a 256 x 256 congestion grid)                    */
 } fx_job_desc;
 typedef struct fx_job_result {
   int64_t job_id, design_id;

@@ -295,7 +295,7 @@ extern "C" int fx_iter_cfg_default(fx_iter_cfg *c) {
   c->density_weight = 1.0e-4f;
   c->target_density = 0.7f;
   c->density_bins = 1024;
-  c->dct_precision = FX_DCT_I8;  // FP32-accurate on the tensor cores; second stream
+  c->dct_precision = FX_DCT_I8;  // FP32-accurate; second stream
   c->cong_cols = 512;
   c->cong_rows = 512;
   c->damping = 0.9f;
@@ -323,9 +323,6 @@ extern "C" int fx_stage_attraction(fx_ctx *ctx, fx_design *d, float k,
 }
 
 namespace fx {
-int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,
-                int precision, bool need_phi, cudaStream_t s);
-
 // A run's statistics and error words, written by one thread straight into
 // the context's pinned readback block: one launch before the final
 // synchronisation instead of a copy per value (and a second round trip for
@@ -657,7 +654,7 @@ extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
   // asynchronous copies; pageable ones would stage through the driver)
   IterReadback &rb = *ctx->readback;
   rb = IterReadback{};
-  const bool tc = use_dens && c.dct_precision != FX_DCT_SIMT;
+  const bool tc = use_dens && c.dct_precision != FX_DCT_SIMT && c.dct_precision != FX_DCT_I8;
   if (iters > 0) {
     iter_stats_kernel<<<1, 32, 0, s>>>(use_cong ? d->cong.result.p : nullptr,
                                        use_cong ? d->cong.result_max.p : nullptr,

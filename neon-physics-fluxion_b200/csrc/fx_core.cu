@@ -468,6 +468,7 @@ extern "C" int fx_design_load(fx_ctx *ctx, int32_t n_gates, int32_t n_nets,
     d->h_w[g] = gate_w ? gate_w[g] : 2.0f;
     d->h_h[g] = gate_h ? gate_h[g] : 10.0f;
     area[g] = d->h_w[g] * d->h_h[g];
+    d->area_sum += (double)area[g];
   }
   const size_t N = (size_t)n_gates;
   auto fail = [&](int code) {

@@ -1,4 +1,4 @@
-// fx_density.cu -- row C: DCT-II Poisson density force as dense GEMM stages.
+// fx_density.cu -- row C: DCT-II Poisson density force.
 //
 // Follows ElectrostaticSmoothingForce (O/src/python/fluxion/
 // force_electrostatic.py):
@@ -12,9 +12,10 @@
 //   field        centred differences inside, one-sided at edges  (:91-103),
 //                applied as the operator products Dx C^T / Dy C^T
 //   force        F_i = area_i * E[row, col] * weight             (:134-150)
-// C is the orthonormal DCT-II matrix (G x G). The transforms are NT GEMMs
-// D = A * B^T with A a constant operator and B the data produced by the
-// previous GEMM (see density_run).
+// C is the orthonormal DCT-II matrix (G x G). The FP32-accurate settings
+// (FX_DCT_SIMT, FX_DCT_I8) solve by fast transforms (fx_dct.cu); the
+// reduced-precision ones by NT GEMMs D = A * B^T with A a constant operator
+// and B the data produced by the previous GEMM (see density_run).
 // Bin areas are accumulated as 64-bit fixed point so the density is exact
 // and independent of the scatter order.
 #include <algorithm>
@@ -22,6 +23,7 @@
 
 #include "fx_internal.h"
 #include "fx_device.cuh"
+#include "fx_dct.cuh"
 #include "fx_gemm.cuh"
 
 namespace fx {
@@ -144,7 +146,7 @@ __global__ void dens_gather_kernel(const float *__restrict__ x,
 }
 
 // Uploads a constant G x G operand computed in FP64 in the formats of
-// `precision`: f32 values (SIMT, TF32), TF32 head + residual (3xTF32), bf16.
+// `precision`: f32 values (TF32), TF32 head + residual (3xTF32), bf16.
 static int upload_operand(const std::vector<double> &m, int precision, float *f32,
                           float *lo, uint16_t *bf, cudaStream_t s) {
   const size_t cells = m.size();
@@ -168,6 +170,46 @@ static int upload_operand(const std::vector<double> &m, int precision, float *f3
   return cudaStreamSynchronize(s) == cudaSuccess ? FX_OK : FX_ECUDA;
 }
 
+// The FP32-accurate settings, solved by fast transforms (fx_dct.cu).
+static bool dct_fast(int precision) {
+  return precision == FX_DCT_SIMT || precision == FX_DCT_I8;
+}
+
+// Tables and grids of the fast-transform solve. wx = 1/bw with bw = die/G
+// (force_electrostatic.py:126-128).
+static int dens_setup_fast(fx_design *d, int G, int precision, cudaStream_t s) {
+  DensityWork &w = d->dens;
+  const size_t cells = (size_t)G * G;
+  const double wx = 1.0 / (double)(d->chip_w / (float)G), wy = 1.0 / (double)(d->chip_h / (float)G);
+  std::vector<double2> tw, qt;
+  std::vector<double> ax2, ay2;
+  dct_tables(G, wx, wy, tw, qt, ax2, ay2);
+  FX_TRY(w.area_fx.alloc(cells));
+  FX_TRY(w.tw.alloc(G));
+  FX_TRY(w.qt.alloc(G));
+  FX_TRY(w.ax2.alloc(G));
+  FX_TRY(w.ay2.alloc(G));
+  FX_TRY(w.buf[1].alloc(cells));  // T1
+  FX_TRY(w.uv.alloc(cells));
+  FX_TRY(w.buf[3].alloc(cells));  // phi
+  FX_TRY(w.ex.alloc(cells));
+  FX_TRY(w.ey.alloc(cells));
+  FX_TRY(w.energy.alloc(4096 + 8));
+  FX_TRY(w.force.alloc((size_t)d->n));
+  const size_t g = (size_t)G;
+  FX_CHECK_CUDA(cudaMemcpyAsync(w.tw.p, tw.data(), g * 16, cudaMemcpyHostToDevice, s));
+  FX_CHECK_CUDA(cudaMemcpyAsync(w.qt.p, qt.data(), g * 16, cudaMemcpyHostToDevice, s));
+  FX_CHECK_CUDA(cudaMemcpyAsync(w.ax2.p, ax2.data(), g * 8, cudaMemcpyHostToDevice, s));
+  FX_CHECK_CUDA(cudaMemcpyAsync(w.ay2.p, ay2.data(), g * 8, cudaMemcpyHostToDevice, s));
+  FX_CHECK_CUDA(cudaMemsetAsync(w.area_fx.p, 0, cells * 8, s));
+  FX_CHECK_CUDA(cudaMemsetAsync(w.energy.p, 0, (4096 + 8) * 8, s));
+  FX_CHECK_CUDA(cudaStreamSynchronize(s));
+  w.halves = false;
+  w.G = G;
+  w.precision = precision;
+  return FX_OK;
+}
+
 // Host: DCT matrix C, the inverse eigenvalues and the field operators
 // Dx C^T, Dy C^T, in FP64 then rounded. Dx is the reference's x stencil
 // (force_electrostatic.py:96-103) as a matrix on a row of phi:
@@ -179,8 +221,9 @@ static int upload_operand(const std::vector<double> &m, int precision, float *f3
 // of a large smooth potential in f32.
 static int dens_setup(fx_design *d, int G, int precision, cudaStream_t s) {
   DensityWork &w = d->dens;
-  if (w.G == G && w.precision == precision && w.cmat.p) return FX_OK;
+  if (w.G == G && w.precision == precision && w.area_fx.p) return FX_OK;
   const size_t cells = (size_t)G * G;
+  if (dct_fast(precision)) return dens_setup_fast(d, G, precision, s);
   FX_TRY(w.area_fx.alloc(cells));
   FX_TRY(w.cmat.alloc(cells));
   FX_TRY(w.cmat_t.alloc(cells));
@@ -197,11 +240,7 @@ static int dens_setup(fx_design *d, int G, int precision, cudaStream_t s) {
   // as E - O, and that difference magnifies the tensor cores' accumulation
   // error (2.1e-4 instead of 5e-5 at G = 256).
   w.halves = G % 256 == 0 && precision != FX_DCT_FP32;
-  {
-    int sp = precision == FX_DCT_SIMT ? sgemm_splits(G, d->ctx->num_sms) : 1;
-    if (w.halves && precision == FX_DCT_SIMT) sp = std::max(sp, half_splits(G, d->ctx->num_sms));
-    if (sp > 1 || w.halves) FX_TRY(w.split_ws.alloc((size_t)sp * cells));
-  }
+  if (w.halves) FX_TRY(w.half_ws.alloc(cells));
   const bool split_fmt = precision == FX_DCT_FP32, bf_fmt = precision == FX_DCT_BF16;
   if (w.halves) {
     FX_TRY(w.c_h.alloc(cells / 2));
@@ -279,50 +318,6 @@ static int dens_setup(fx_design *d, int G, int precision, cudaStream_t s) {
       ie[(size_t)ky * G + kx] = (kx == 0 && ky == 0) ? 0.0f : (float)(-1.0 / lam);
     }
   FX_CHECK_CUDA(cudaMemcpyAsync(w.inv_eig.p, ie.data(), cells * 4, cudaMemcpyHostToDevice, s));
-  // FX_DCT_I8: the operators' 8-bit slices, cut from their FP64 values (7
-  // bits of each row's scale per slice), in the order [s1 ..] along NS K
-  // columns, for rows x K operators (the full G x G ones, or the 2 x (G/2) x
-  // (G/2) half operators below)
-  auto slice_op = [&](const std::vector<double> &m, int rows, int K, int o) -> int {
-    const int NS = i8_slices();
-    std::vector<int8_t> sl((size_t)NS * rows * K);
-    std::vector<float> sc(rows);
-    for (int i = 0; i < rows; ++i) {
-      double mx = 0.0;
-      for (int k = 0; k < K; ++k) mx = std::max(mx, std::fabs(m[(size_t)i * K + k]));
-      int e = 0;
-      if (mx > 0.0) std::frexp(mx, &e);
-      sc[i] = std::ldexp(1.0f, e);
-      for (int k = 0; k < K; ++k) {
-        double a = std::ldexp(m[(size_t)i * K + k], -e);
-        for (int t = 0; t < NS; ++t) {
-          const double q = a * 128.0;
-          const double tr = std::trunc(q);
-          sl[(size_t)i * NS * K + (size_t)t * K + k] = (int8_t)tr;
-          a = q - tr;
-        }
-      }
-    }
-    FX_TRY(w.op8[o].alloc(sl.size()));
-    FX_TRY(w.op_sc[o].alloc(rows));
-    FX_CHECK_CUDA(cudaMemcpyAsync(w.op8[o].p, sl.data(), sl.size(), cudaMemcpyHostToDevice, s));
-    FX_CHECK_CUDA(cudaMemcpyAsync(w.op_sc[o].p, sc.data(), (size_t)rows * 4,
-                                  cudaMemcpyHostToDevice, s));
-    FX_CHECK_CUDA(cudaStreamSynchronize(s));  // sl and sc go out of scope
-    return FX_OK;
-  };
-  if (precision == FX_DCT_I8) {
-    for (int i = 0; i < 2; ++i) {  // data slices: G x NS G (or 2G x NS G/2)
-      FX_TRY(w.d8[i].alloc((size_t)i8_slices() * cells));
-      FX_TRY(w.d_sc[i].alloc(2 * (size_t)G));
-    }
-    if (!w.halves) {
-      FX_TRY(slice_op(c, G, G, 0));
-      FX_TRY(slice_op(ct, G, G, 1));
-      FX_TRY(slice_op(dx, G, G, 2));
-      FX_TRY(slice_op(dy, G, G, 3));
-    }
-  }
   FX_TRY(upload_operand(c, precision, w.cmat.p, split ? w.cmat_lo.p : nullptr,
                         half ? w.cmat_bf.p : nullptr, s));
   FX_TRY(upload_operand(ct, precision, w.cmat_t.p, split ? w.cmat_t_lo.p : nullptr,
@@ -357,12 +352,6 @@ static int dens_setup(fx_design *d, int G, int precision, cudaStream_t s) {
                           bf_fmt ? w.dx_h_bf.p : nullptr, s));
     FX_TRY(upload_operand(dyh, precision, w.dy_h.p, split_fmt ? w.dy_h_lo.p : nullptr,
                           bf_fmt ? w.dy_h_bf.p : nullptr, s));
-    if (precision == FX_DCT_I8) {  // the two halves of each, as 2h rows of h
-      FX_TRY(slice_op(chh, 2 * h, h, 0));
-      FX_TRY(slice_op(cth, 2 * h, h, 1));
-      FX_TRY(slice_op(dxh, 2 * h, h, 2));
-      FX_TRY(slice_op(dyh, 2 * h, h, 3));
-    }
   }
   FX_CHECK_CUDA(cudaMemsetAsync(w.area_fx.p, 0, cells * 8, s));
   FX_CHECK_CUDA(cudaMemsetAsync(w.energy.p, 0, (4096 + 8) * 8, s));
@@ -395,8 +384,10 @@ int density_scatter(fx_ctx *ctx, fx_design *d, const float *x, const float *y,
 //   T1^T = C rho^T ; phi_hat = (C T1) * (-1/lambda) ;
 //   T3^T = C^T phi_hat^T ; E_y = (Dy C^T) T3 ;
 //   T4^T = (Dx C^T) phi_hat^T ; E_x = C^T T4 ; [phi = C^T T3].
+// The FP32-accurate settings take the same map by fast transforms instead;
+// rho_out (their charge grid in f32, or null) is for callers that return it.
 int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,
-                int precision, bool need_phi, cudaStream_t s) {
+                int precision, bool need_phi, cudaStream_t s, float *rho_out) {
   (void)weight;
   FX_TRY(dens_setup(d, G, precision, s));
   DensityWork &w = d->dens;
@@ -405,6 +396,29 @@ int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,
   const double inv_bin_area = 1.0 / ((double)bw * (double)bh);
   cudaEvent_t ev;
   timer_begin(ctx, FX_STAGE_DENSITY, s, &ev);
+  if (dct_fast(precision)) {
+    DctArgs a{};
+    a.G = G;
+    a.acc = w.area_fx.p;
+    a.inv_bin_area = inv_bin_area;
+    a.target = (double)target;
+    a.level = d->area_sum * inv_bin_area / ((double)G * (double)G);
+    a.wx = 1.0 / (double)bw;
+    a.wy = 1.0 / (double)bh;
+    a.tw = w.tw.p;
+    a.qt = w.qt.p;
+    a.ax2 = w.ax2.p;
+    a.ay2 = w.ay2.p;
+    a.rho = rho_out;
+    a.t1 = w.buf[1].p;
+    a.uv = w.uv.p;
+    a.ex = w.ex.p;
+    a.ey = w.ey.p;
+    a.phi = need_phi ? w.buf[3].p : nullptr;
+    FX_TRY(dct_solve(ctx, a, s));
+    timer_end(ctx, FX_STAGE_DENSITY, s, ev);
+    return FX_OK;
+  }
   const int eb = ctx->num_sms * 8;
   // Split (3xTF32) and bf16 operand copies exist only for their precision.
   const bool split = precision == FX_DCT_FP32, half = precision == FX_DCT_BF16;
@@ -417,33 +431,6 @@ int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,
       w.area_fx.p, cells, inv_bin_area, target, w.buf[0].p, LO(2), BF(0));
   FX_CHECK_LAUNCH();
   ctx->launches += 1;
-  float *WS = precision == FX_DCT_SIMT ? w.split_ws.p : nullptr;
-  if (precision == FX_DCT_I8 && !w.halves) {
-    // the same seven products; each data operand is sliced once and kept
-    // while later products read it (phat and T3 twice)
-    float *rho = w.buf[0].p, *t1 = w.buf[1].p, *phat = w.buf[2].p, *t3 = w.buf[1].p;
-    float *t4 = w.buf[4].p;
-    auto slice = [&](const float *X, int i) {
-      return i8_slice(ctx, X, G, G, w.d8[i].p, w.d_sc[i].p, s);
-    };
-    auto mm = [&](int op, int i, const float *S, float *D) {
-      return gemm_nt_i8(ctx, G, w.op8[op].p, w.op_sc[op].p, w.d8[i].p, w.d_sc[i].p, S, D, s);
-    };
-    FX_TRY(slice(rho, 0));
-    FX_TRY(mm(0, 0, nullptr, t1));              // T1^T = C rho^T
-    FX_TRY(slice(t1, 0));
-    FX_TRY(mm(0, 0, w.inv_eig.p, phat));        // phi_hat = (C T1) * (-1/lambda)
-    FX_TRY(slice(phat, 1));
-    FX_TRY(mm(1, 1, nullptr, t3));              // T3^T = C^T phi_hat^T
-    FX_TRY(slice(t3, 0));
-    FX_TRY(mm(3, 0, nullptr, w.ey.p));          // E_y = (Dy C^T) T3
-    if (need_phi) FX_TRY(mm(1, 0, nullptr, w.buf[3].p));  // phi = C^T T3
-    FX_TRY(mm(2, 1, nullptr, t4));              // T4^T = (Dx C^T) phi_hat^T
-    FX_TRY(slice(t4, 0));
-    FX_TRY(mm(1, 0, nullptr, w.ex.p));          // E_x = C^T T4
-    timer_end(ctx, FX_STAGE_DENSITY, s, ev);
-    return FX_OK;
-  }
   if (w.halves) {
     // each product as two half-size GEMMs on the folded or split operand;
     // products come back as f32 and the folds write the GEMM formats
@@ -465,30 +452,7 @@ int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,
     const GemmOperands Dyh = K(w.dy_h.p, w.dy_h_lo.p, w.dy_h_bf.p);
     float *rho = w.buf[0].p, *t1 = w.buf[1].p, *phat = w.buf[2].p, *t3 = w.buf[1].p;
     float *t4 = w.buf[4].p, *phi = w.buf[3].p;
-    float *P = w.split_ws.p;
-    if (precision == FX_DCT_I8) {
-      // the same products from 8-bit slices; each folded or split operand
-      // is sliced by its product (into d8[0] / d_sc[0])
-      auto hm = [&](int op, int i, int mode, float sign, const float *S, float *D) {
-        return gemm_half_i8(ctx, G, w.op8[op].p, w.op_sc[op].p, w.hw[i].p, mode, sign, S, D, P,
-                            w.d8[0].p, w.d_sc[0].p, s);
-      };
-      fold(rho, H(0));
-      FX_TRY(hm(0, 0, kHalfRows, 1.f, nullptr, t1));
-      fold(t1, H(0));
-      FX_TRY(hm(0, 0, kHalfRows, 1.f, w.inv_eig.p, phat));
-      split_k(phat, H(1));
-      FX_TRY(hm(1, 1, kHalfPair, 1.f, nullptr, t3));
-      split_k(t3, H(2));
-      FX_TRY(hm(3, 2, kHalfPair, -1.f, nullptr, w.ey.p));
-      if (need_phi) FX_TRY(hm(1, 2, kHalfPair, 1.f, nullptr, phi));
-      FX_TRY(hm(2, 1, kHalfPair, -1.f, nullptr, t4));
-      split_k(t4, H(0));
-      FX_TRY(hm(1, 0, kHalfPair, 1.f, nullptr, w.ex.p));
-      FX_CHECK_LAUNCH();
-      timer_end(ctx, FX_STAGE_DENSITY, s, ev);
-      return FX_OK;
-    }
+    float *P = w.half_ws.p;
     fold(rho, H(0));
     FX_TRY(gemm_half(ctx, precision, G, Ch, H(0), kHalfRows, 1.f, nullptr, t1, P, s));
     fold(t1, H(0));
@@ -518,13 +482,13 @@ int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,
   const GemmOperands ex{w.ex.p, nullptr, nullptr};
   const GemmOperands ey{w.ey.p, nullptr, nullptr};
   const GemmOperands phi{w.buf[3].p, nullptr, nullptr};
-  FX_TRY(gemm_nt(ctx, precision, G, C, rho, nullptr, t1, s, WS));
-  FX_TRY(gemm_nt(ctx, precision, G, C, t1, w.inv_eig.p, phat, s, WS));
-  FX_TRY(gemm_nt(ctx, precision, G, Ct, phat, nullptr, t3, s, WS));
-  FX_TRY(gemm_nt(ctx, precision, G, DyCt, t3, nullptr, ey, s, WS));
-  if (need_phi) FX_TRY(gemm_nt(ctx, precision, G, Ct, t3, nullptr, phi, s, WS));
-  FX_TRY(gemm_nt(ctx, precision, G, DxCt, phat, nullptr, t4, s, WS));
-  FX_TRY(gemm_nt(ctx, precision, G, Ct, t4, nullptr, ex, s, WS));
+  FX_TRY(gemm_nt(ctx, precision, G, C, rho, nullptr, t1, s));
+  FX_TRY(gemm_nt(ctx, precision, G, C, t1, w.inv_eig.p, phat, s));
+  FX_TRY(gemm_nt(ctx, precision, G, Ct, phat, nullptr, t3, s));
+  FX_TRY(gemm_nt(ctx, precision, G, DyCt, t3, nullptr, ey, s));
+  if (need_phi) FX_TRY(gemm_nt(ctx, precision, G, Ct, t3, nullptr, phi, s));
+  FX_TRY(gemm_nt(ctx, precision, G, DxCt, phat, nullptr, t4, s));
+  FX_TRY(gemm_nt(ctx, precision, G, Ct, t4, nullptr, ex, s));
   timer_end(ctx, FX_STAGE_DENSITY, s, ev);
   return FX_OK;
 }
@@ -564,7 +528,9 @@ extern "C" int fx_stage_density(fx_ctx *ctx, fx_design *d, int32_t bins,
   cudaStream_t s = ctx->stream;
   const float *x = d->x[d->cur].p, *y = d->y[d->cur].p;
   FX_TRY(density_scatter(ctx, d, x, y, bins, precision, s));
-  FX_TRY(density_run(ctx, d, bins, target_density, weight, precision, true, s));
+  if (out_rho) FX_TRY(d->dens.buf[0].alloc((size_t)bins * bins));
+  FX_TRY(density_run(ctx, d, bins, target_density, weight, precision, true, s,
+                     out_rho ? d->dens.buf[0].p : nullptr));
   FX_TRY(density_gather(ctx, d, x, y, bins, weight, s));
   DensityWork &w = d->dens;
   const size_t cells = (size_t)bins * bins, n = (size_t)d->n;

@@ -184,8 +184,8 @@ struct DensityWork {
   DevBuf<float> ex, ey;                // field
   DevBuf<double> energy;               // FP64 partials
   DevBuf<float2> force;                // per gate
-  DevBuf<float> split_ws;              // SIMT split-K partial tiles
-  // even/odd path (G a multiple of 256): the half operators
+  DevBuf<float> half_ws;               // half products before their placing
+  // even/odd GEMMs (G a multiple of 256): the half operators
   // [C even rows | C odd rows], [C^T even cols | odd cols], Dx C^T, Dy C^T
   // likewise, each (G/2) x (G/2) pair in one buffer of G*G/2; and three
   // folded or split data operands of G*G each
@@ -195,10 +195,11 @@ struct DensityWork {
   DevBuf<uint16_t> c_h_bf, ct_h_bf, dx_h_bf, dy_h_bf;   // bf16 copies
   DevBuf<float> hw[3], hw_lo[3];
   DevBuf<uint16_t> hw_bf[3];
-  // FX_DCT_I8: 8-bit slices (G x 4G) and row scales of the operators C, C^T,
-  // Dx C^T, Dy C^T, and of two data operands at a time
-  DevBuf<int8_t> op8[4], d8[2];
-  DevBuf<float> op_sc[4], d_sc[2];
+  // fast transforms (FX_DCT_SIMT, FX_DCT_I8; fx_dct.cu): tables and the
+  // (u, Dy u) grid between the column and row passes
+  DevBuf<double2> tw, qt;
+  DevBuf<double> ax2, ay2;
+  DevBuf<float2> uv;
   template <class F>
   void for_each(F &&f) {
     f(area_fx); f(cmat); f(cmat_t); f(cmat_lo); f(cmat_t_lo); f(cmat_bf);
@@ -207,17 +208,14 @@ struct DensityWork {
     for (auto &b : buf) f(b);
     for (auto &b : lo) f(b);
     for (auto &b : bf) f(b);
-    f(ex); f(ey); f(energy); f(force); f(split_ws);
+    f(ex); f(ey); f(energy); f(force); f(half_ws);
     f(c_h); f(ct_h); f(dx_h); f(dy_h);
     f(c_h_lo); f(ct_h_lo); f(dx_h_lo); f(dy_h_lo);
     f(c_h_bf); f(ct_h_bf); f(dx_h_bf); f(dy_h_bf);
     for (auto &b : hw) f(b);
     for (auto &b : hw_lo) f(b);
     for (auto &b : hw_bf) f(b);
-    for (auto &b : op8) f(b);
-    for (auto &b : d8) f(b);
-    for (auto &b : op_sc) f(b);
-    for (auto &b : d_sc) f(b);
+    f(tw); f(qt); f(ax2); f(ay2); f(uv);
   }
 };
 
@@ -294,6 +292,7 @@ struct fx_design {
   fx::DevBuf<int32_t> net_ptr, net_gate;
   fx::DevBuf<int32_t> adj_ptr, adj_idx;
   fx::DevBuf<float> area;        // w*h per gate
+  double area_sum = 0.0;         // of all gates
   std::vector<int32_t> h_adj_ptr, h_adj_idx;
   std::vector<float> h_w, h_h;
   // state: ping-pong positions, velocities
@@ -356,7 +355,7 @@ int attraction_run(fx_ctx *ctx, fx_design *d, float k, float2 *out, cudaStream_t
 int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int walk,
            cudaStream_t s, int32_t *term_count = nullptr);
 int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,
-                int precision, bool need_phi, cudaStream_t s);
+                int precision, bool need_phi, cudaStream_t s, float *rho_out = nullptr);
 int fused_step(fx_ctx *ctx, fx_design *d, const fx_iter_cfg &cfg,
                cudaStream_t s);
 // Stable LSD radix sort of (key, value) pairs (fx_bh.cu).
