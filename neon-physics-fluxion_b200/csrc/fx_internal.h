@@ -255,6 +255,7 @@ struct IterReadback {
   float max_overflow;
   unsigned int err;     // Barnes-Hut error word
   unsigned int tc_err;  // tensor-core GEMM error word
+  uint32_t refine[2][8];  // fx_refine's loop state, one slot per iteration parity
 };
 
 }  // namespace fx
