@@ -42,6 +42,7 @@
 #include <cstdlib>
 
 #include "fx_internal.h"
+#include "fx_bh.cuh"
 #include "fx_device.cuh"
 
 namespace fx {
@@ -98,47 +99,18 @@ __global__ void bh_bbox_kernel(const float *__restrict__ x,
   }
 }
 
-// Root square from the box (BarnesHutTree.cpp:24-46, in f32 without
-// contraction), then re-arms the box for the next accumulation.
+// Root square of the box, then re-arms the box for the next accumulation.
 __global__ void bh_root_kernel(unsigned int *__restrict__ bbox,
                                float *__restrict__ root, float th2, float md2) {
-  float mnx = ord2f(bbox[0]), mny = ord2f(bbox[1]);
-  float mxx = ord2f(bbox[2]), mxy = ord2f(bbox[3]);
-  mnx = __fsub_rn(mnx, 1.0f);
-  mxx = __fadd_rn(mxx, 1.0f);
-  mny = __fsub_rn(mny, 1.0f);
-  mxy = __fadd_rn(mxy, 1.0f);
-  const float size = fmaxf(__fsub_rn(mxx, mnx), __fsub_rn(mxy, mny));
-  const float cx = __fmul_rn(__fadd_rn(mnx, mxx), 0.5f);
-  const float cy = __fmul_rn(__fadd_rn(mny, mxy), 0.5f);
-  const float half = __fmul_rn(size, 0.5f);
-  root[0] = __fsub_rn(cx, half);
-  root[1] = __fsub_rn(cy, half);
-  root[2] = size;
-  // deep keys when a level-15 cell is not always accepted
-  const float s15 = ldexpf(size, -15);
-  root[3] = __fmul_rn(s15, s15) >= __fmul_rn(th2, md2) ? 1.0f : 0.0f;
+  const float4 r = bh_root_of(bbox, th2, md2);
+  root[0] = r.x;
+  root[1] = r.y;
+  root[2] = r.z;
+  root[3] = r.w;
   bbox[0] = 0xffffffffu;
   bbox[1] = 0xffffffffu;
   bbox[2] = 0u;
   bbox[3] = 0u;
-}
-
-__device__ __forceinline__ uint32_t quantize15(float p, float o, float size) {
-  const float t = __fmul_rn(__fdiv_rn(__fsub_rn(p, o), size), 32768.0f);
-  if (!(t > 0.0f)) return 0u;
-  const float c = ceilf(t);
-  if (c >= 32768.0f) return 32767u;
-  return (uint32_t)c - 1u;
-}
-
-__device__ __forceinline__ uint32_t spread15(uint32_t v) {
-  v &= 0x7fffu;
-  v = (v | (v << 8)) & 0x00ff00ffu;
-  v = (v | (v << 4)) & 0x0f0f0f0fu;
-  v = (v | (v << 2)) & 0x33333333u;
-  v = (v | (v << 1)) & 0x55555555u;
-  return v;
 }
 
 // Sub-cell (0..4095) of p within its level-15 cell c15, in f64 without
@@ -617,63 +589,6 @@ int radix_sort_onesweep(uint32_t *k[2], int32_t *v[2], int n, int passes, uint32
   return FX_OK;
 }
 
-// ---- radix tree (Karras 2012) -----------------------------------------------
-// Common prefix length of the keys at sorted positions i and j: 30-bit key,
-// then (deep mode, lo != null) the 24-bit sub-key, then the index.
-__device__ __forceinline__ int bh_delta(const uint32_t *__restrict__ keys,
-                                        const uint32_t *__restrict__ lo,
-                                        int n, int i, int j) {
-  if (j < 0 || j >= n) return -1;
-  const uint32_t a = keys[i], b = keys[j];
-  if (a != b) return __clz(a ^ b) - 2;
-  if (lo) {
-    const uint32_t la = lo[i], lb = lo[j];
-    if (la != lb) return kKeyBits + __clz(la ^ lb) - 8;
-    return kDeepBits + __clz((uint32_t)(i ^ j));
-  }
-  return kKeyBits + __clz((uint32_t)(i ^ j));
-}
-
-__global__ void bh_tree_kernel(const uint32_t *__restrict__ keys,
-                               const uint32_t *__restrict__ slo,
-                               const float *__restrict__ root, int n,
-                               int32_t *__restrict__ child,
-                               int32_t *__restrict__ range,
-                               int32_t *__restrict__ dnode,
-                               int32_t *__restrict__ dparent) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n - 1) return;
-  const uint32_t *sub = (slo && root[3] > 0.f) ? slo : nullptr;
-  const int dr = bh_delta(keys, sub, n, i, i + 1), dl = bh_delta(keys, sub, n, i, i - 1);
-  const int d = (dr - dl) >= 0 ? 1 : -1;
-  const int dmin = bh_delta(keys, sub, n, i, i - d);
-  int lmax = 2;
-  while (bh_delta(keys, sub, n, i, i + lmax * d) > dmin) lmax *= 2;
-  int l = 0;
-  for (int t = lmax / 2; t >= 1; t /= 2)
-    if (bh_delta(keys, sub, n, i, i + (l + t) * d) > dmin) l += t;
-  const int j = i + l * d;
-  const int dn = bh_delta(keys, sub, n, i, j);
-  int s = 0;
-  for (int div = 2;; div *= 2) {
-    const int t = (l + div - 1) / div;
-    if (bh_delta(keys, sub, n, i, i + (s + t) * d) > dn) s += t;
-    if (t == 1) break;
-  }
-  const int gamma = i + s * d + min(d, 0);
-  const int lo = min(i, j), hi = max(i, j);
-  const int left = (lo == gamma) ? ~gamma : gamma;
-  const int right = (hi == gamma + 1) ? ~(gamma + 1) : gamma + 1;
-  child[2 * i] = left;
-  child[2 * i + 1] = right;
-  range[2 * i] = lo;
-  range[2 * i + 1] = hi;
-  dnode[i] = dn;
-  if (left >= 0) dparent[left] = dn;
-  if (right >= 0) dparent[right] = dn;
-  if (i == 0) dparent[0] = -1;
-}
-
 // ---- exact prefix sums of the sorted positions ---------------------------------
 // Every position becomes the 128-bit integer trunc(v * 2^64) (exact for
 // |v| >= 2^-41; smaller magnitudes lose their bits below 2^-64, non-finite
@@ -684,30 +599,6 @@ __global__ void bh_tree_kernel(const uint32_t *__restrict__ keys,
 // with hi/lo the upper (signed) and lower (unsigned) 64 bits, each step
 // rounded to nearest.
 constexpr int kFixThreads = 256, kFixItems = 8, kFixTile = kFixThreads * kFixItems;
-
-__device__ __forceinline__ __int128 fixed64(float v) {
-  const uint32_t u = __float_as_uint(v);
-  const int e = (int)((u >> 23) & 255u);
-  if (e == 0 || e == 255) return 0;
-  const unsigned long long m = (u & 0x7fffffu) | 0x800000u;  // v = m * 2^(e - 150)
-  const int sh = e - 86;                                     // v * 2^64 = m * 2^(e - 86)
-  unsigned __int128 r = 0;
-  if (sh >= 0) r = (unsigned __int128)m << sh;
-  else if (sh > -64) r = m >> (-sh);
-  return (u >> 31) ? -(__int128)r : (__int128)r;
-}
-
-__device__ __forceinline__ ulonglong2 pack128(__int128 v) {
-  return make_ulonglong2((unsigned long long)v, (unsigned long long)((unsigned __int128)v >> 64));
-}
-__device__ __forceinline__ __int128 unpack128(ulonglong2 p) {
-  return (__int128)(((unsigned __int128)p.y << 64) | p.x);
-}
-__device__ __forceinline__ __int128 shfl_up128(__int128 v, int d) {
-  const ulonglong2 p = pack128(v);
-  return unpack128(make_ulonglong2(__shfl_up_sync(0xffffffffu, p.x, d),
-                                   __shfl_up_sync(0xffffffffu, p.y, d)));
-}
 
 // Inclusive scan of one int128 per thread over the block; also returns the
 // block total.
@@ -732,81 +623,78 @@ __device__ __forceinline__ __int128 block_scan128(__int128 v, __int128 &total) {
   return v + off;
 }
 
-// Pass 1: the (x, y) sums of each tile of kFixTile sorted points.
+// The (x, y) sums of each tile of kFixTile sorted points.
 __global__ void __launch_bounds__(kFixThreads)
 fix_tile_kernel(const float2 *__restrict__ spos, int n, ulonglong4 *__restrict__ tile_sum) {
-  const int b0 = blockIdx.x * kFixTile + threadIdx.x * kFixItems;
-  __int128 sx = 0, sy = 0;
+  const int b0 = blockIdx.x * kFixTile + threadIdx.x;
+  FixSums s{0, 0};
 #pragma unroll
   for (int k = 0; k < kFixItems; ++k) {
-    const int i = b0 + k;
+    const int i = b0 + k * kFixThreads;
     if (i < n) {
       const float2 p = spos[i];
-      sx += fixed64(p.x);
-      sy += fixed64(p.y);
+      s.x += fixed64(p.x);
+      s.y += fixed64(p.y);
     }
   }
-  __int128 tx, ty;
-  block_scan128(sx, tx);
-  block_scan128(sy, ty);
-  if (threadIdx.x == 0) {
-    const ulonglong2 a = pack128(tx), c = pack128(ty);
-    tile_sum[blockIdx.x] = make_ulonglong4(a.x, a.y, c.x, c.y);
-  }
+  s = block_sums128<kFixThreads>(s);
+  if (threadIdx.x == 0) tile_sum[blockIdx.x] = pack_sums(s);
 }
 
-// Pass 2: exclusive offsets of the tiles (one block, kFixThreads tiles at a
-// time, carrying the running total; exact, so the grouping is free).
-__global__ void __launch_bounds__(kFixThreads)
-fix_top_kernel(ulonglong4 *__restrict__ tile_sum, int tiles) {
-  __int128 cx = 0, cy = 0;
-  for (int base = 0; base < tiles; base += kFixThreads) {
-    const int t = base + threadIdx.x;
-    __int128 vx = 0, vy = 0;
-    if (t < tiles) {
-      const ulonglong4 v = tile_sum[t];
-      vx = unpack128(make_ulonglong2(v.x, v.y));
-      vy = unpack128(make_ulonglong2(v.z, v.w));
-    }
-    __int128 tx, ty;
-    const __int128 ix = block_scan128(vx, tx);
-    const __int128 iy = block_scan128(vy, ty);
-    if (t < tiles) {
-      const ulonglong2 a = pack128(cx + ix - vx), c = pack128(cy + iy - vy);
-      tile_sum[t] = make_ulonglong4(a.x, a.y, c.x, c.y);
-    }
-    cx += tx;
-    cy += ty;
-  }
-}
-
-// Pass 3: inclusive prefix of every point (x lo/hi, y lo/hi).
+// Inclusive prefix of every point (x lo/hi, y lo/hi), tiles of 256 * kItems
+// points: a block adds up the sums of all earlier tiles itself (they are few
+// and in L2; a scan of them would be another launch), then scans its own. A
+// thread's points are consecutive; they and the prefixes pass through shared
+// memory, each warp's by itself, so that global accesses coalesce. 23 us with
+// the tile sums at 1M points, 8 at 5k (31 and 17 with their scan, each thread
+// writing its own run of 32-byte prefixes).
+template <int kItems>
 __global__ void __launch_bounds__(kFixThreads)
 fix_prefix_kernel(const float2 *__restrict__ spos, int n,
-                  const ulonglong4 *__restrict__ tile_off, ulonglong4 *__restrict__ prefix) {
-  const int b0 = blockIdx.x * kFixTile + threadIdx.x * kFixItems;
-  __int128 sx = 0, sy = 0;
+                  const ulonglong4 *__restrict__ tile_sum, ulonglong4 *__restrict__ prefix) {
+  constexpr int kWarps = kFixThreads / 32, kRun = 32 * kItems;  // points of a warp
+  constexpr int kHalf = 2;  // of a thread's points, staged per turn
+  __shared__ float2 pts[kWarps][kRun + 32];
+  __shared__ ulonglong4 out[kWarps][32 * kHalf + 32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int w0 = blockIdx.x * (kFixThreads * kItems) + w * kRun;
 #pragma unroll
-  for (int k = 0; k < kFixItems; ++k) {
-    const int i = b0 + k;
-    if (i < n) {
-      const float2 p = spos[i];
-      sx += fixed64(p.x);
-      sy += fixed64(p.y);
-    }
+  for (int k = 0; k < kItems; ++k) {
+    const int j = k * 32 + lane;
+    pts[w][j + j / kItems] = w0 + j < n ? spos[w0 + j] : make_float2(0.f, 0.f);
   }
-  __int128 tx, ty;
-  const ulonglong4 to = tile_off[blockIdx.x];
-  __int128 rx = block_scan128(sx, tx) - sx + unpack128(make_ulonglong2(to.x, to.y));
-  __int128 ry = block_scan128(sy, ty) - sy + unpack128(make_ulonglong2(to.z, to.w));
-  for (int k = 0; k < kFixItems; ++k) {  // the points again (cached), in order
-    const int i = b0 + k;
-    if (i >= n) break;
-    const float2 p = spos[i];
-    rx += fixed64(p.x);
-    ry += fixed64(p.y);
-    const ulonglong2 a = pack128(rx), c = pack128(ry);
-    prefix[i] = make_ulonglong4(a.x, a.y, c.x, c.y);
+  FixSums off{0, 0};
+  for (int q = t; q < (int)blockIdx.x; q += kFixThreads) {
+    const FixSums v = unpack_sums(tile_sum[q]);
+    off.x += v.x;
+    off.y += v.y;
+  }
+  off = block_sums128<kFixThreads>(off);
+  __syncwarp();
+  FixSums p[kItems], s{0, 0};
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) {
+    const float2 v = pts[w][lane * (kItems + 1) + k];
+    s.x += fixed64(v.x);
+    s.y += fixed64(v.y);
+    p[k] = s;
+  }
+  FixSums tot;
+  off.x += block_scan128(s.x, tot.x) - s.x;
+  off.y += block_scan128(s.y, tot.y) - s.y;
+#pragma unroll
+  for (int h = 0; h < kItems; h += kHalf) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k)
+      out[w][lane * (kHalf + 1) + k] = pack_sums({off.x + p[h + k].x, off.y + p[h + k].y});
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k) {
+      const int j = k * 32 + lane;  // the j-th staged prefix: lane j / kHalf's
+      const int i = w0 + (j / kHalf) * kItems + h + j % kHalf;
+      if (i < n) prefix[i] = out[w][j + j / kHalf];
+    }
   }
 }
 
@@ -819,29 +707,127 @@ __device__ __forceinline__ double fixed_to_double(__int128 v) {
                    5.42101086242752217003726400434970855712890625e-20);
 }
 
+// ---- radix tree (Karras 2012) and walk records --------------------------------
+// One thread per internal node does everything the walk needs of it: its
+// range and split, its centre of mass from the prefix sums, and its quad
+// children. What it needs of its parent is the larger of the two prefix lengths
+// at its range's ends; what it needs of a child is that child's own prefix
+// length and, where the child stands for no quad level, its split, which the
+// warp mostly has (shuffles; the few large nodes search). One launch instead
+// of two with ranges, splits and lengths stored between them: 14 us against
+// 15 at 5k points (ncu cold) and a launch less in the chain; about even at 1M
+// (67 us against 60). Latency of the searches' loads and divergence bound it
+// (14 of 32 lanes active).
+constexpr int kBuildThreads = 256;
+
+struct BhKeys {
+  const uint32_t *keys, *lo;  // sorted keys; sub-keys (deep mode) or null
+  int n;
+  __device__ __forceinline__ uint32_t at(int i) const { return __ldg(keys + i); }
+  // Common prefix length of the keys a, b at sorted positions i and j: 30-bit
+  // key, then (deep mode) the 24-bit sub-key, then the index.
+  __device__ __forceinline__ int delta_of(uint32_t a, uint32_t b, int i, int j) const {
+    if (a != b) return __clz(a ^ b) - 2;
+    if (lo) {
+      const uint32_t la = lo[i], lb = lo[j];
+      if (la != lb) return kKeyBits + __clz(la ^ lb) - 8;
+      return kDeepBits + __clz((uint32_t)(i ^ j));
+    }
+    return kKeyBits + __clz((uint32_t)(i ^ j));
+  }
+  __device__ __forceinline__ int delta(int i, int j) const {
+    return j < 0 || j >= n ? -1 : delta_of(at(i), at(j), i, j);
+  }
+  // The largest x in [lo_x, hi_x] with delta(i, i + x d) > thr, which holds at
+  // lo_x and stops holding once. Ranges beyond the staged keys take seven
+  // probes a step, their loads in flight together (the chain of a binary
+  // search in global memory is most of this kernel's time on small designs);
+  // the short ranges of almost all nodes are bisected, since there the
+  // instructions count (105 us at 1M points with seven probes throughout).
+  __device__ __forceinline__ int reach(int i, int d, int lo_x, int hi_x, int thr) const {
+    const uint32_t a = at(i);
+    while (hi_x - lo_x > 64) {
+      const int step = (hi_x - lo_x + 8) >> 3;  // eight parts of [lo_x, hi_x]
+      uint32_t b[7];
+#pragma unroll
+      for (int p = 0; p < 7; ++p) b[p] = __ldg(keys + (i + min(lo_x + (p + 1) * step, hi_x) * d));
+      int c = 0;
+#pragma unroll
+      for (int p = 0; p < 7; ++p) {
+        const int x = lo_x + (p + 1) * step;
+        if (x <= hi_x && delta_of(a, b[p], i, i + x * d) > thr) c = p + 1;
+      }
+      lo_x += c * step;
+      hi_x = min(hi_x, lo_x + step - 1);
+    }
+    while (hi_x > lo_x) {
+      const int x = (lo_x + hi_x + 1) >> 1;
+      if (delta_of(a, at(i + x * d), i, i + x * d) > thr) lo_x = x;
+      else hi_x = x - 1;
+    }
+    return lo_x;
+  }
+  // Last place of the left child of the node [f, l] with prefix length dn.
+  __device__ __forceinline__ int split(int f, int l, int dn) const {
+    return f + reach(f, 1, 0, l - f - 1, dn);
+  }
+};
+
+constexpr int kNone = INT_MIN;
+
 // Walk record of every internal node (two float4):
 //   r0 = {cx_hi, cy_hi, cx_lo, cy_lo}  centre of mass as an f32 hi/lo pair
 //   r1 = {count (negative: bucket), size^2 (negative: no quad level),
 //         first, last (as int bits)}
-__device__ __forceinline__ void bh_qchild(int i, const int32_t *__restrict__ child,
-                                          const int32_t *__restrict__ dnode, int kb,
-                                          int4 *__restrict__ qchild);
-
-// Also writes the node's quad children (bh_qchild below).
-__global__ void bh_node_kernel(int n, const int32_t *__restrict__ range,
-                               const int32_t *__restrict__ dnode,
-                               const int32_t *__restrict__ dparent,
-                               const ulonglong4 *__restrict__ prefix,
-                               const float *__restrict__ root, int deep_ok,
-                               float4 *__restrict__ node,
-                               const int32_t *__restrict__ child,
-                               int4 *__restrict__ qchild) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n - 1) return;
-  bh_qchild(i, child, dnode, (deep_ok && root[3] > 0.f) ? kDeepBits : kKeyBits, qchild);
-  const bool deep = deep_ok && root[3] > 0.f;
+// and its quad children: a child that stands for no quad level (at most one
+// such level separates two quad cells) is replaced by its own two children, so
+// every node lists up to four, in key order (leaf s as ~s, kNone: empty).
+__global__ void __launch_bounds__(kBuildThreads)
+bh_build_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ slo,
+                const float *__restrict__ root, int n,
+                const ulonglong4 *__restrict__ prefix, float4 *__restrict__ node,
+                int4 *__restrict__ qchild) {
+  const int i = blockIdx.x * kBuildThreads + threadIdx.x;
+  const bool valid = i < n - 1;
+  const bool deep = slo && root[3] > 0.f;
   const int kb = deep ? kDeepBits : kKeyBits;  // prefix length of a bucket
-  const int f = range[2 * i], l = range[2 * i + 1];
+  const BhKeys k{keys, deep ? slo : nullptr, n};
+  int f = 0, l = 0, dn = 0, dp = 0, gamma = 0;
+  if (valid) {
+    // range: extends from i toward the neighbour it shares more with
+    const int dr = k.delta(i, i + 1), dl = k.delta(i, i - 1);
+    const int d = (dr - dl) >= 0 ? 1 : -1;
+    const int dmin = min(dr, dl);
+    // grow the range by factors of two, past 64 of eight, then search the last
+    const int most = d > 0 ? n - 1 - i : i;  // places on that side
+    int in = 1, top = min(2, most);          // holds at in; unknown at top
+    while (top > in && k.delta(i, i + top * d) > dmin) {
+      const int by = top < 64 ? 2 : 8;
+      in = top;
+      top = top > most / by ? most : top * by;
+    }
+    const int j = i + k.reach(i, d, in, top, dmin) * d;
+    f = min(i, j);
+    l = max(i, j);
+    dn = k.delta(i, j);
+    // the parent's prefix length: at i's end it is dmin, at the other end it is
+    // what the node shares with the next place
+    dp = max(dmin, d > 0 ? k.delta(l, l + 1) : k.delta(f, f - 1));
+    gamma = k.split(f, l, dn);
+  }
+  // the children's prefix lengths and splits, from the lanes that have them
+  // (small nodes: a child's index is close to its parent's)
+  const int base = i & ~31;
+  int cdn[2], cgam[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int src = gamma + h - base;
+    cdn[h] = __shfl_sync(0xffffffffu, dn, src & 31);
+    cgam[h] = __shfl_sync(0xffffffffu, gamma, src & 31);
+    if ((unsigned)src >= 32u) cgam[h] = -1;
+  }
+  if (!valid) return;
+  // centre of mass
   const int cnt = l - f + 1;
   const ulonglong4 pl = prefix[l];
   __int128 sx = unpack128(make_ulonglong2(pl.x, pl.y));
@@ -851,11 +837,31 @@ __global__ void bh_node_kernel(int n, const int32_t *__restrict__ range,
     sx -= unpack128(make_ulonglong2(pf.x, pf.y));
     sy -= unpack128(make_ulonglong2(pf.z, pf.w));
   }
+  int out[4] = {kNone, kNone, kNone, kNone};
+  int o = 0;
+  const int lv = dn >> 1;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int cf = h ? gamma + 1 : f, cl = h ? l : gamma;
+    if (cf == cl) {
+      out[o++] = ~cf;
+      continue;
+    }
+    const int ci = gamma + h;
+    const int dc = cgam[h] >= 0 ? cdn[h] : k.delta(cf, cl);
+    if (dc < kb && (dc >> 1) == lv) {
+      const int g = cgam[h] >= 0 ? cgam[h] : k.split(cf, cl, dc);
+      out[o++] = g == cf ? ~g : g;
+      out[o++] = g + 1 == cl ? ~(g + 1) : g + 1;
+    } else {
+      out[o++] = ci;
+    }
+  }
+  qchild[i] = make_int4(out[0], out[1], out[2], out[3]);
   const double cx = __ddiv_rn(fixed_to_double(sx), (double)cnt);
   const double cy = __ddiv_rn(fixed_to_double(sy), (double)cnt);
   const float hx = (float)cx, hy = (float)cy;
   node[2 * i] = make_float4(hx, hy, (float)(cx - (double)hx), (float)(cy - (double)hy));
-  const int dn = dnode[i], dp = dparent[i];
   const float rs = root[2];
   float c, s2;
   if (dn >= kb) {
@@ -863,40 +869,15 @@ __global__ void bh_node_kernel(int n, const int32_t *__restrict__ range,
     c = -(float)cnt;
     s2 = __fmul_rn(sz, sz);
   } else {
-    const int lmax = dn >> 1;
     c = (float)cnt;
-    if (dp >= 0 && (dp >> 1) == lmax) {
+    if (dp >= 0 && (dp >> 1) == lv) {
       s2 = -1.0f;
     } else {
-      const float sz = ldexpf(rs, -lmax);
+      const float sz = ldexpf(rs, -lv);
       s2 = __fmul_rn(sz, sz);
     }
   }
   node[2 * i + 1] = make_float4(c, s2, __int_as_float(f), __int_as_float(l));
-}
-
-// Quad children: a node that stands for no quad level (at most one such level
-// separates two quad cells) is replaced by its own two children, so every
-// node lists up to four children, in key order. kNone marks empty slots.
-constexpr int kNone = INT_MIN;
-
-__device__ __forceinline__ void bh_qchild(int i, const int32_t *__restrict__ child,
-                                          const int32_t *__restrict__ dnode, int kb,
-                                          int4 *__restrict__ qchild) {
-  int out[4] = {kNone, kNone, kNone, kNone};
-  int k = 0;
-  const int lv = dnode[i] >> 1;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int c = child[2 * i + h];
-    if (c >= 0 && dnode[c] < kb && (dnode[c] >> 1) == lv) {
-      out[k++] = child[2 * c];
-      out[k++] = child[2 * c + 1];
-    } else {
-      out[k++] = c;
-    }
-  }
-  qchild[i] = make_int4(out[0], out[1], out[2], out[3]);
 }
 
 // ---- warp-cooperative walk ----------------------------------------------------
@@ -1285,12 +1266,8 @@ static int bh_alloc(fx_design *d) {
   FX_TRY(b.tile_scan.alloc((size_t)256 * T));
   FX_TRY(b.digit_total.alloc(256));
   FX_TRY(b.spos.alloc(n));
-  FX_TRY(b.child.alloc(2 * ni));
-  FX_TRY(b.range.alloc(2 * ni));
-  FX_TRY(b.dnode.alloc(ni));
-  FX_TRY(b.dparent.alloc(ni));
   FX_TRY(b.qchild.alloc(ni));
-  FX_TRY(b.tile_fix.alloc((size_t)(n + kFixTile - 1) / kFixTile));
+  FX_TRY(b.tile_fix.alloc(std::max(((size_t)n + kFixTile - 1) / kFixTile, (size_t)64)));
   FX_TRY(b.prefix.alloc(n));
   FX_TRY(b.node.alloc(2 * ni));
   FX_TRY(b.root.alloc(4));
@@ -1353,22 +1330,15 @@ int bh_bbox(fx_ctx *ctx, fx_design *d, const float *x, const float *y,
   return FX_OK;
 }
 
-// Full Barnes-Hut force evaluation on the current positions; bh.bbox must
-// hold their bounding box. Result: bh.force (original gate order).
-int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int walk,
-           cudaStream_t s, int32_t *term_count) {
-  FX_TRY(bh_alloc(d));
+// Keys, sort and sorted positions of a design of any size (with the deep-key
+// kernels when `deep`), by kernels of many blocks.
+static int bh_sort_large(fx_ctx *ctx, fx_design *d, const float *x, const float *y, float th2,
+                         float md2, bool deep, cudaStream_t s) {
   BHWork &b = d->bh;
-  const int n = d->n;
-  const float *x = d->x[d->cur].p, *y = d->y[d->cur].p;
+  const int n = d->n, gb = (n + 255) / 256;
   const int T = (n + kSortTile - 1) / kSortTile;
-  unsigned int *err = b.bbox.p + 4;
-  const float th2 = theta * theta, md2 = min_dist * min_dist;
-  const bool deep = bh_maybe_deep(d, th2, md2);  // launch the deep-key kernels
-  if (deep) FX_TRY(bh_alloc_deep(d));
-  cudaEvent_t ev;
-  const int gb = (n + 255) / 256;
   int launches = 0;
+  cudaEvent_t ev;
   timer_begin(ctx, FX_STAGE_BH_KEYS, s, &ev);
   bh_root_kernel<<<1, 1, 0, s>>>(b.bbox.p, b.root.p, th2, md2);
   FX_CHECK_LAUNCH();
@@ -1404,7 +1374,7 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
     uint32_t *kk[2] = {b.keys[0].p, b.keys[1].p};
     int32_t *vv[2] = {b.idx[0].p, b.idx[1].p};
     // result in buffer 0; the last pass also gathers the sorted positions
-    FX_TRY(radix_sort_onesweep(kk, vv, n, 4, b.os_ws.p, err, s, x, y, b.spos.p));
+    FX_TRY(radix_sort_onesweep(kk, vv, n, 4, b.os_ws.p, b.bbox.p + 4, s, x, y, b.spos.p));
   }
   launches += 5;
   if (deep) {
@@ -1413,20 +1383,53 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
   }
   FX_CHECK_LAUNCH();
   timer_end(ctx, FX_STAGE_BH_SORT, s, ev);
+  ctx->launches += launches;
+  return FX_OK;
+}
+
+// Full Barnes-Hut force evaluation on the current positions; bh.bbox must
+// hold their bounding box. Result: bh.force (original gate order).
+int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int walk,
+           cudaStream_t s, int32_t *term_count) {
+  FX_TRY(bh_alloc(d));
+  BHWork &b = d->bh;
+  const int n = d->n;
+  const float *x = d->x[d->cur].p, *y = d->y[d->cur].p;
+  unsigned int *err = b.bbox.p + 4;
+  const float th2 = theta * theta, md2 = min_dist * min_dist;
+  const bool deep = bh_maybe_deep(d, th2, md2);  // launch the deep-key kernels
+  if (deep) FX_TRY(bh_alloc_deep(d));
+  cudaEvent_t ev;
+  int launches = 0;
+  // Small designs: one cluster does keys and sort (fx_bh_sort.cu) up to its
+  // capacity: 20 us at 5k points and 28 at 10k against 69 and 73 for the seven
+  // launches of the many-block kernels.
+  const bool one = !deep && n <= bh_cluster_max();
+  if (one) {
+    timer_begin(ctx, FX_STAGE_BH_SORT, s, &ev);
+    FX_TRY(bh_cluster_sort(ctx, x, y, n, b.bbox.p, th2, md2, b.keys[0].p, b.idx[0].p, b.spos.p,
+                           b.tile_fix.p, b.root.p, s));
+    timer_end(ctx, FX_STAGE_BH_SORT, s, ev);
+  } else {
+    FX_TRY(bh_sort_large(ctx, d, x, y, th2, md2, deep, s));
+  }
   timer_begin(ctx, FX_STAGE_BH_TREE, s, &ev);
   if (n >= 2) {
-    const int tb = (n - 1 + 255) / 256;
-    bh_tree_kernel<<<tb, 256, 0, s>>>(b.keys[0].p, deep ? b.slo.p : nullptr, b.root.p, n,
-                                      b.child.p, b.range.p, b.dnode.p, b.dparent.p);
-    // exact prefix sums: tile sums, tile offsets, point prefixes
-    const int tiles = (n + kFixTile - 1) / kFixTile;
-    fix_tile_kernel<<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p);
-    fix_top_kernel<<<1, kFixThreads, 0, s>>>(b.tile_fix.p, tiles);
-    fix_prefix_kernel<<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p, b.prefix.p);
-    bh_node_kernel<<<tb, 256, 0, s>>>(n, b.range.p, b.dnode.p, b.dparent.p,
-                                      b.prefix.p, b.root.p, deep ? 1 : 0, b.node.p, b.child.p,
-                                      b.qchild.p);
-    launches += 5;
+    // exact prefix sums, from tile sums (the cluster sort makes its own)
+    if (one) {
+      fix_prefix_kernel<2><<<(n + 511) / 512, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p,
+                                                                   b.prefix.p);
+    } else {
+      const int tiles = (n + kFixTile - 1) / kFixTile;
+      fix_tile_kernel<<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p);
+      fix_prefix_kernel<kFixItems><<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p,
+                                                                 b.prefix.p);
+      ++launches;
+    }
+    ++launches;
+    bh_build_kernel<<<(n - 1 + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s>>>(
+        b.keys[0].p, deep ? b.slo.p : nullptr, b.root.p, n, b.prefix.p, b.node.p, b.qchild.p);
+    ++launches;
   }
   FX_CHECK_LAUNCH();
   timer_end(ctx, FX_STAGE_BH_TREE, s, ev);

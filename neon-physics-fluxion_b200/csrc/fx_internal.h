@@ -136,12 +136,8 @@ struct BHWork {
   DevBuf<uint32_t> tile_scan;   // per-digit exclusive scan of tile_hist
   DevBuf<uint32_t> digit_total; // 256 digit totals
   DevBuf<float2> spos;          // positions in sorted order
-  DevBuf<int32_t> child;        // internal nodes: 2 children (leaf s -> ~s)
-  DevBuf<int32_t> range;        // internal nodes: first, last
-  DevBuf<int32_t> dnode;        // internal nodes: prefix length
-  DevBuf<int32_t> dparent;      // internal nodes: parent's prefix length
   DevBuf<int4> qchild;          // internal nodes: up to 4 quad children
-  DevBuf<ulonglong4> tile_fix;  // per-tile exact (x, y) sums, then offsets
+  DevBuf<ulonglong4> tile_fix;  // per-tile exact (x, y) sums
   DevBuf<ulonglong4> prefix;    // inclusive exact prefix sums of spos (2 x int128)
   DevBuf<float4> node;          // internal nodes: 2 x float4 walk records
   DevBuf<float> root;           // {x_min, y_min, size, deep (1) or not (0)}
@@ -158,8 +154,8 @@ struct BHWork {
     f(os_ws);
     for (auto &b : keys) f(b);
     for (auto &b : idx) f(b);
-    f(tile_hist); f(tile_scan); f(digit_total); f(spos); f(child); f(range);
-    f(dnode); f(dparent); f(qchild); f(klo); f(kl[0]); f(kl[1]); f(il[0]); f(il[1]); f(slo);
+    f(tile_hist); f(tile_scan); f(digit_total); f(spos);
+    f(qchild); f(klo); f(kl[0]); f(kl[1]); f(il[0]); f(il[1]); f(slo);
     f(tile_fix); f(prefix); f(node); f(root); f(bbox); f(force);
   }
 };
