@@ -1080,20 +1080,31 @@ bh_walk_kernel(int n, const float2 *__restrict__ spos,
 // ---- batched walk (FX_BH_FAST) ----------------------------------------------
 // The same cells, decisions and terms as the group walk, organised by cell
 // instead of by point. Each warp owns 32 consecutive sorted points and a
-// stack of (cell, lane mask) entries: the cells opened by at least one of
-// its points, with the lanes that must evaluate them. A pass pops up to 32
-// entries, one per lane; each lane loads its entry's walk record into shared
-// memory, then every lane evaluates all popped entries for its own point
-// (broadcast reads), adds the accepted terms and votes which lanes open each
-// entry. Opened cells push their quad children with that vote as the mask;
-// opened buckets are walked point by point. Every lane does the same work in
-// every step (no divergence between cells, points and buckets), and a cell
-// is loaded once per warp instead of once per group. Per point the
-// interaction list is exactly the group walk's (the same opening rule with
-// the same f32 operations); the terms are added in another order.
-// The stack holds kBatchStack entries (the 1M-gate uniform placement peaks at
-// 219; clustered, line and radial sets of 20k-200k points at 160-224 in a CPU
-// model of this walk): a warp whose stack would overflow starts over with
+// stack of opened cells: the quad children of each, and the lanes that opened
+// it and so must evaluate them. A pass pops up to eight cells, a child per
+// lane (popping single children instead costs a 32-lane scan of four ids per
+// push); each lane first settles its entry for all 32 points at once from the
+// box around them:
+//   * accepted by all (the opening rule holds at the box's nearest point, with
+//     a margin for the rounding of the per-point test; or a single point):
+//     its term is added without any test, two entries per packed f32x2
+//     instruction (entries that only some lanes must evaluate: one at a time,
+//     masked);
+//   * opened by all (the rule fails at the farthest point): its children are
+//     pushed with its mask, and nothing is evaluated;
+//   * neither: every lane evaluates it for its own point from broadcast reads,
+//     adds the term if it accepts and votes who opens it, with the f32
+//     operations of the group walk.
+// Opened cells push their quad children with the opening lanes as the mask;
+// opened buckets are walked point by point. Per point the interaction list is
+// exactly the group walk's; the terms are added in another order.
+// Issue-bound (78 % issue-active, ALU pipe 63 %): of the 613 entries of a warp
+// at 1M uniform points 125 are accepted by all, 272 by a mask, 159 tested and
+// 57 opened by all; testing every entry for every lane took 0.66 ms and
+// 604M warp instructions, this 0.57 ms and 476M (300k points: 0.217, 0.198 ms).
+// The stack holds kBatchStack cells (of up to four children; in a CPU model
+// of this walk the children of uniform, clustered, line and radial sets of
+// 20k-1M points peaked at 160-224): a warp whose stack would overflow starts over with
 // the group walk, whose stacks are bounded, in the same shared memory.
 // The hardware reciprocal square root without the subnormal handling of
 // rsqrtf (the argument here is at least min_dist^2).
@@ -1104,11 +1115,9 @@ __device__ __forceinline__ float rsqrt_approx_ftz(float x) {
 }
 
 constexpr int kBatchWarps = 8;
-constexpr int kBatchStack = 400;
-static_assert(kBatchStack * sizeof(int2) >= 2 * kWalkGroups * (kStackDeep + 1) * sizeof(int32_t),
-              "the group walk's stacks must fit in a warp's batch stack");
+constexpr int kBatchStack = 200;
 
-// The stack entries a warp may use (kBatchStack; less when the environment
+// The stacked cells a warp may use (kBatchStack; less when the environment
 // variable FLUXION_BH_BATCH_STACK asks for it, a test setting that sends more
 // warps down the group-walk path).
 static int batch_stack_cap() {
@@ -1120,6 +1129,53 @@ static int batch_stack_cap() {
   return cap;
 }
 
+// Packed pairs of f32 (one instruction, each half rounded as the scalar one).
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Two entries side by side, one half of each packed register: -x and -y of
+// their centres (head and tail), k * mass, lane mask, size^2. 80 bytes, so
+// that the lanes' stores to their halves conflict two ways at most.
+struct alignas(16) EntryPair {
+  uint64_t xh, yh;
+  uint64_t xl, yl;
+  uint64_t m, mask;
+  uint64_t s2, self;  // self: (counting) the point of a single-point entry
+  uint64_t pad[2];
+};
+
+struct BatchSmem {
+  int4 kids[kBatchStack];      // an opened cell's quad children
+  unsigned mask[kBatchStack];  // and the lanes that opened it
+  EntryPair rec[16];           // the entries of a pass, two by two
+  unsigned open_s[32];         // per entry: the lanes opening it
+};
+static_assert(kBatchStack * sizeof(int4) >= 2 * kWalkGroups * (kStackDeep + 1) * sizeof(int32_t),
+              "the group walk's stacks must fit in a warp's batch stack");
+
 template <int Stack, bool Count>
 __global__ void __launch_bounds__(kBatchWarps * 32, 5)
 bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__restrict__ perm,
@@ -1127,83 +1183,186 @@ bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__re
                      float k, float th2, float md2, float2 *__restrict__ force,
                      unsigned int *__restrict__ err, int32_t *__restrict__ term_count,
                      int stack_cap) {
-  __shared__ int2 st[kBatchWarps][kBatchStack];
-  __shared__ float4 rec_a[kBatchWarps][32];  // cx_hi, cy_hi, cx_lo, cy_lo
-  __shared__ float4 rec_b[kBatchWarps][32];  // k*mass, size^2 rule, lane mask, self
-  __shared__ unsigned open_s[kBatchWarps][32];  // per popped entry: the lanes opening it
+  __shared__ __align__(16) BatchSmem smem[kBatchWarps];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const bool lane0 = lane == 0;
+  BatchSmem &sh = smem[w];
   const int base = (blockIdx.x * kBatchWarps + w) * 32;
   if (base >= n) return;  // warp-uniform
   const int s = base + lane;
   const bool valid = s < n;
-  const unsigned lanebit = 1u << lane;
+  const unsigned lanebit = 1u << lane, lt = lanebit - 1u;
   const float2 p = valid ? spos[s] : make_float2(0.f, 0.f);
+  const unsigned vm = __ballot_sync(full, valid);
+  // the points' box: centre and half extents, grown by the rounding of both
+  // and of the per-point differences; with a non-finite point nothing is
+  // settled for all (the comparisons with an infinite extent fail)
+  float bcx, bcy, bhx, bhy;
+  {
+    const float2 q = valid ? p : spos[base];
+    float x0 = q.x, x1 = q.x, y0 = q.y, y1 = q.y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      x0 = fminf(x0, __shfl_xor_sync(full, x0, o));
+      x1 = fmaxf(x1, __shfl_xor_sync(full, x1, o));
+      y0 = fminf(y0, __shfl_xor_sync(full, y0, o));
+      y1 = fmaxf(y1, __shfl_xor_sync(full, y1, o));
+    }
+    bcx = 0.5f * x0 + 0.5f * x1;
+    bcy = 0.5f * y0 + 0.5f * y1;
+    const float slack = 1e-6f * (fmaxf(fabsf(x0), fabsf(x1)) + fmaxf(fabsf(y0), fabsf(y1)));
+    bhx = 0.5f * (x1 - x0) + slack;
+    bhy = 0.5f * (y1 - y0) + slack;
+    if (!__all_sync(full, isfinite(q.x) && isfinite(q.y))) bhx = bhy = __int_as_float(0x7f800000);
+  }
+  const float th2md2 = __fmul_rn(th2, md2);
+  const float th2_lo = th2 * 0.999f, th2_hi = th2 * 1.001f;
+  const uint64_t px2 = pack2(p.x, p.x), py2 = pack2(p.y, p.y);
+  uint64_t fx2 = 0, fy2 = 0;
   float fx = 0.f, fy = 0.f;
   int terms = 0;
-  int sp = 0;  // stack depth (warp-uniform)
+  int sp = 0;  // opened cells on the stack (warp-uniform)
+  // the first pass evaluates the root alone, as the only child of a cell that
+  // every point opened
   if (n >= 2) {
-    const unsigned vm = __ballot_sync(full, valid);
-    if (lane == 0) st[w][0] = make_int2(0, (int)vm);
+    if (lane == 0) {
+      sh.kids[0] = make_int4(0, kNone, kNone, kNone);
+      sh.mask[0] = vm;
+    }
     sp = 1;
   }
   __syncwarp();
   bool overflow = false;
   while (sp > 0) {
-    const int cnt = min(sp, 32);
+    // pop up to eight opened cells: lane l takes child l % 4 of cell l / 4
+    const int cnt = min(sp, 8);
     sp -= cnt;
     int c = kNone, bf = 0, bl = -1;
-    bool bucket = false;
-    if (lane < cnt) {
-      const int2 e = st[w][sp + lane];
-      c = e.x;
-      float4 a, b;
-      if (c >= 0) {
-        a = node[2 * c];
-        const float4 r1 = node[2 * c + 1];
-        // size^2 < 0 (a node standing for no quad level): never accepted
-        b = make_float4(__fmul_rn(k, fabsf(r1.x)), r1.y >= 0.f ? r1.y : __int_as_float(0x7f800000),
-                        __int_as_float(e.y), __int_as_float(-1));
-        bucket = !(r1.x > 0.f);
-        bf = __float_as_int(r1.z);
-        bl = __float_as_int(r1.w);
-      } else {  // single point ~c: always accepted
-        const float2 q = spos[~c];
-        a = make_float4(q.x, q.y, 0.f, 0.f);
-        b = make_float4(k, -1.f, __int_as_float(e.y), __int_as_float(~c));
+    unsigned mask = 0u;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    float kq = 0.f, s2 = 0.f;
+    bool bucket = false, all_acc = false, all_open = false;
+    if (lane < 4 * cnt) {
+      c = reinterpret_cast<const int *>(sh.kids + sp)[lane];
+      mask = sh.mask[sp + (lane >> 2)];
+    }
+    const bool has = c != kNone;
+    if (c >= 0) {
+      a = node[2 * c];
+      const float4 r1 = node[2 * c + 1];
+      // size^2 < 0 (a node standing for no quad level): never accepted
+      kq = __fmul_rn(k, fabsf(r1.x));
+      s2 = r1.y >= 0.f ? r1.y : __int_as_float(0x7f800000);
+      bucket = !(r1.x > 0.f);
+      bf = __float_as_int(r1.z);
+      bl = __float_as_int(r1.w);
+      // squared distances from the centre of mass to the box's nearest and
+      // farthest points
+      const float ax = fabsf(a.x - bcx), ay = fabsf(a.y - bcy);
+      const float slack = 1e-6f * (fabsf(a.x) + fabsf(a.y));
+      const float nx = fmaxf(ax - bhx - slack, 0.f), ny = fmaxf(ay - bhy - slack, 0.f);
+      const float qx = ax + bhx + slack, qy = ay + bhy + slack;
+      all_acc = s2 < th2md2 || s2 < th2_lo * (nx * nx + ny * ny);
+      all_open = !all_acc && s2 >= th2_hi * fmaxf(qx * qx + qy * qy, md2);
+    } else if (has) {  // single point ~c: always accepted
+      const float2 q = spos[~c];
+      a = make_float4(q.x, q.y, 0.f, 0.f);
+      kq = k;
+      s2 = -1.f;
+      all_acc = true;
+    }
+    // staged in one run: accepted by all, accepted by the lanes of a mask, to
+    // be tested. A pair that straddles two kinds is treated as the later one,
+    // which is right for both.
+    const bool staged = has && !all_open;
+    const unsigned b_all = __ballot_sync(full, all_acc && mask == vm);
+    const unsigned b_acc = __ballot_sync(full, all_acc);
+    const unsigned b_any = __ballot_sync(full, staged);
+    const int n_all = __popc(b_all), n_acc = __popc(b_acc), n_any = __popc(b_any);
+    int slot = 0;
+    if (staged) {
+      const unsigned bit = lanebit;
+      slot = (b_all & bit) ? __popc(b_all & lt)
+             : (b_acc & bit) ? n_all + __popc((b_acc & ~b_all) & lt)
+                             : n_acc + __popc((b_any & ~b_acc) & lt);
+      float *r = reinterpret_cast<float *>(&sh.rec[slot >> 1]) + (slot & 1);
+      r[0] = -a.x;
+      r[2] = -a.y;
+      r[4] = -a.z;
+      r[6] = -a.w;
+      r[8] = kq;
+      r[10] = __uint_as_float(mask);
+      r[12] = s2;
+      if (Count) r[14] = __int_as_float(c < 0 ? ~c : -1);
+      if (slot + 1 == n_any && !(slot & 1)) {  // fill the last pair
+        r[1] = r[3] = r[5] = r[7] = r[9] = r[11] = r[13] = 0.f;
+        if (Count) r[15] = __int_as_float(-1);
       }
-      rec_a[w][lane] = a;
-      rec_b[w][lane] = b;
     }
     __syncwarp();
-#pragma unroll 4
-    for (int j = 0; j < cnt; ++j) {
-      const float4 a = rec_a[w][j];
-      const float4 b = rec_b[w][j];
-      const float dx = __fsub_rn(__fsub_rn(p.x, a.x), a.z);
-      const float dy = __fsub_rn(__fsub_rn(p.y, a.y), a.w);
-      const float r2c = fmaxf(__fmaf_rn(dx, dx, __fmul_rn(dy, dy)), md2);
-      const bool in = (__float_as_uint(b.z) & lanebit) != 0u;
-      const bool acc = b.y < __fmul_rn(th2, r2c);
-      const unsigned om = __ballot_sync(full, in && !acc);
-      if (lane0) open_s[w][j] = om;
-      const float inv = rsqrt_approx_ftz(r2c);  // r2c >= md2 > 0: never subnormal
-      const float f = __fmul_rn(__fmul_rn(__fmul_rn(b.x, inv), inv), inv);
-      const float fu = (in && acc) ? f : 0.f;
-      fx = __fmaf_rn(fu, dx, fx);
-      fy = __fmaf_rn(fu, dy, fy);
-      if (Count) terms += (in && acc && __float_as_int(b.w) != s) ? 1 : 0;
+    // both entries' differences and squared distances
+    auto pair_r = [&](const EntryPair &q, uint64_t &dx, uint64_t &dy) {
+      dx = add2(add2(px2, q.xh), q.xl);
+      dy = add2(add2(py2, q.yh), q.yl);
+      const float2 r2 = unpack2(fma2(dx, dx, mul2(dy, dy)));
+      return make_float2(fmaxf(r2.x, md2), fmaxf(r2.y, md2));
+    };
+    // their terms; m: k * mass, 0 where a lane takes none
+    auto pair_add = [&](uint64_t m, float2 r2c, uint64_t dx, uint64_t dy) {
+      // r2c >= md2 > 0: never subnormal
+      const uint64_t inv = pack2(rsqrt_approx_ftz(r2c.x), rsqrt_approx_ftz(r2c.y));
+      const uint64_t f = mul2(mul2(mul2(m, inv), inv), inv);
+      fx2 = fma2(f, dx, fx2);
+      fy2 = fma2(f, dy, fy2);
+    };
+    int j = 0;
+#pragma unroll 2
+    for (; j < (n_all >> 1); ++j) {
+      const EntryPair &q = sh.rec[j];
+      uint64_t dx, dy;
+      const float2 r2c = pair_r(q, dx, dy);
+      pair_add(q.m, r2c, dx, dy);
+      if (Count) terms += ((int)(uint32_t)q.self != s) + ((int)(q.self >> 32) != s);
+    }
+#pragma unroll 2
+    for (; j < (n_acc >> 1); ++j) {
+      const EntryPair &q = sh.rec[j];
+      uint64_t dx, dy;
+      const float2 r2c = pair_r(q, dx, dy);
+      const float2 m = unpack2(q.m);
+      const bool in0 = ((uint32_t)q.mask & lanebit) != 0u;
+      const bool in1 = ((uint32_t)(q.mask >> 32) & lanebit) != 0u;
+      pair_add(pack2(in0 ? m.x : 0.f, in1 ? m.y : 0.f), r2c, dx, dy);
+      if (Count)
+        terms += (in0 && (int)(uint32_t)q.self != s) + (in1 && (int)(q.self >> 32) != s);
+    }
+#pragma unroll 2
+    for (; 2 * j < n_any; ++j) {
+      const EntryPair &q = sh.rec[j];
+      uint64_t dx, dy;
+      const float2 r2c = pair_r(q, dx, dy);
+      const float2 m = unpack2(q.m), sq = unpack2(q.s2);
+      const bool in0 = ((uint32_t)q.mask & lanebit) != 0u;
+      const bool in1 = ((uint32_t)(q.mask >> 32) & lanebit) != 0u;
+      const bool acc0 = sq.x < __fmul_rn(th2, r2c.x), acc1 = sq.y < __fmul_rn(th2, r2c.y);
+      const unsigned o0 = __ballot_sync(full, in0 && !acc0);
+      const unsigned o1 = __ballot_sync(full, in1 && !acc1);
+      if (lane == 0) reinterpret_cast<uint64_t *>(sh.open_s)[j] = (uint64_t)o1 << 32 | o0;
+      pair_add(pack2(in0 && acc0 ? m.x : 0.f, in1 && acc1 ? m.y : 0.f), r2c, dx, dy);
+      if (Count)
+        terms += (in0 && acc0 && (int)(uint32_t)q.self != s) +
+                 (in1 && acc1 && (int)(q.self >> 32) != s);
     }
     __syncwarp();
-    const unsigned myopen = lane < cnt ? open_s[w][lane] : 0u;
+    // the lanes that open this lane's cell
+    const unsigned myopen = all_open ? mask : (staged && !all_acc) ? sh.open_s[slot] : 0u;
     // opened buckets: their points one by one
     unsigned bk = __ballot_sync(full, bucket && myopen != 0u);
     while (bk) {
-      const int j = __ffs(bk) - 1;
+      const int b = __ffs(bk) - 1;
       bk &= bk - 1u;
-      const unsigned om = __shfl_sync(full, myopen, j);
-      const int f = __shfl_sync(full, bf, j), l = __shfl_sync(full, bl, j);
+      const unsigned om = __shfl_sync(full, myopen, b);
+      const int f = __shfl_sync(full, bf, b), l = __shfl_sync(full, bl, b);
       const bool in = (om & lanebit) != 0u;
       for (int t = f; t <= l; ++t) {
         const float2 q = spos[t];
@@ -1214,32 +1373,24 @@ bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__re
       }
     }
     // opened cells: push their quad children with the opening lanes as mask
-    const bool op = myopen != 0u && c >= 0 && !bucket;
-    int4 q = make_int4(kNone, kNone, kNone, kNone);
-    if (op) q = qchild[c];
-    const int nc = (q.x != kNone) + (q.y != kNone) + (q.z != kNone) + (q.w != kNone);
-    int incl = nc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(full, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const int total = __shfl_sync(full, incl, 31);
+    const bool op = myopen != 0u && !bucket;
+    const unsigned b_op = __ballot_sync(full, op);
+    const int total = __popc(b_op);
     if (sp + total > stack_cap) {  // stack_cap <= kBatchStack
       overflow = true;
       break;
     }
-    int pos = sp + incl - nc;
-    const int qc[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int h = 0; h < 4; ++h)
-      if (qc[h] != kNone) st[w][pos++] = make_int2(qc[h], (int)myopen);
+    if (op) {
+      const int at = sp + __popc(b_op & lt);
+      sh.kids[at] = qchild[c];
+      sh.mask[at] = myopen;
+    }
     sp += total;
     __syncwarp();
   }
   if (overflow) {  // warp-uniform: start over with the bounded group walk
     __syncwarp();
-    int32_t *mem = reinterpret_cast<int32_t *>(&st[w][0]);
+    int32_t *mem = reinterpret_cast<int32_t *>(&sh.kids[0]);
     bh_group_walk<Stack, true, Count>(
         base, n, spos, perm, qchild, node, k, th2, md2, force, err, term_count,
         reinterpret_cast<int32_t(*)[Stack + 1]>(mem),
@@ -1247,7 +1398,8 @@ bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__re
     return;
   }
   if (valid) {
-    force[perm[s]] = make_float2(fx, fy);
+    const float2 ax = unpack2(fx2), ay = unpack2(fy2);
+    force[perm[s]] = make_float2(fx + (ax.x + ax.y), fy + (ay.x + ay.y));
     if (Count) term_count[perm[s]] = terms;
   }
 }
