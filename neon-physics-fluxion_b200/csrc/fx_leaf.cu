@@ -43,7 +43,7 @@ struct LeafBatch {
   const int32_t *gptr;     // [L+1] offsets into the gate list (leaf order)
   const int32_t *gate;     // [G] global gate ids; ~gate for a slot whose gate a
                            // later slot of the batch writes again
-  const int32_t *aptr;     // [G+1] in-leaf adjacency row offsets
+  const int32_t *abeg, *aend;  // [G] in-leaf adjacency rows
   const int16_t *aidx;     // in-leaf neighbour local indices (reference order)
   const float4 *region;    // [L] (cx, cy, w, h)
   const int32_t *order;    // [L] leaves in processing order
@@ -119,7 +119,7 @@ __device__ void place_leaf(const LeafBatch &b, int leaf, int tid, float *sm, int
     for (int i = tid; i < n; i += T) {
       const float xi = sx[i], yi = sy[i];
       float ax = 0.f, ay = 0.f;
-      const int a0 = b.aptr[g0 + i], a1 = b.aptr[g0 + i + 1];
+      const int a0 = b.abeg[g0 + i], a1 = b.aend[g0 + i];
       for (int e = a0; e < a1; ++e) {
         const int j = b.aidx[e];
         ax = __fadd_rn(ax, __fmul_rn(b.k, __fsub_rn(sx[j], xi)));
@@ -287,7 +287,7 @@ __device__ void place_leaf_pairs(const LeafBatch &b, int leaf, int nmax, float2 
       float ax = 0.f, ay = 0.f;
       if (j < n) {
         const float2 pj = sxy[j];
-        const int a0 = b.aptr[g0 + j], a1 = b.aptr[g0 + j + 1];
+        const int a0 = b.abeg[g0 + j], a1 = b.aend[g0 + j];
         for (int e = a0; e < a1; ++e) {
           const float2 po = sxy[b.aidx[e]];
           ax = __fadd_rn(ax, __fmul_rn(b.k, __fsub_rn(po.x, pj.x)));
@@ -520,12 +520,89 @@ static int launch_pairs(fx_ctx *ctx, const LeafBatch &b, const PairPlan &plan, c
   return FX_OK;
 }
 
-// Host-side leaf structures: in-leaf adjacency in the reference's order and
-// a largest-first processing order.
+// Leaves largest first, in leaf order among equals (sizes 0 .. kLeafMax).
+static std::vector<int32_t> leaf_order(int L, const int32_t *leaf_ptr) {
+  std::vector<int32_t> at(kLeafMax + 2, 0), order(L);
+  auto key = [&](int l) { return kLeafMax - (leaf_ptr[l + 1] - leaf_ptr[l]); };
+  for (int l = 0; l < L; ++l) ++at[key(l) + 1];
+  for (int k = 0; k <= kLeafMax; ++k) at[k + 1] += at[k];
+  for (int l = 0; l < L; ++l) order[at[key(l)]++] = l;
+  return order;
+}
+
+// ---- in-leaf adjacency on the device -------------------------------------------
+// For batches that list every gate at most once (all that a hierarchy makes):
+// slot i's row holds the local indices of the neighbours of its gate that lie
+// in the same leaf, in the design's adjacency order. Built on the host, by up
+// to 16 threads, this took most of a call (16 of 19 ms for 16,384 leaves,
+// whose kernel runs 3 ms).
+
+// map[g] = slot of gate g (-1 before); flag: 1 a gate out of range, 2 a gate
+// listed twice.
+__global__ void leaf_map_kernel(const int32_t *__restrict__ gate, int G, int n,
+                                int32_t *__restrict__ map, unsigned int *__restrict__ flag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= G) return;
+  const int g = gate[i];
+  if (g < 0 || g >= n) atomicOr(flag, 1u);
+  else if (atomicExch(map + g, i) != -1) atomicOr(flag, 2u);
+}
+
+// A warp per leaf: counts its gates' in-leaf neighbours, takes the leaf's
+// share of aidx from *total (rows of a leaf are dense and in slot order; where
+// the leaf's share lies depends on timing, what it holds does not), writes them.
+__global__ void __launch_bounds__(256)
+leaf_adj_kernel(int L, const int32_t *__restrict__ gptr, const int32_t *__restrict__ gate,
+                const int32_t *__restrict__ map, const int32_t *__restrict__ adj_ptr,
+                const int32_t *__restrict__ adj_idx, unsigned int *__restrict__ total,
+                int32_t *__restrict__ abeg, int32_t *__restrict__ aend,
+                int16_t *__restrict__ aidx) {
+  const int l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (l >= L) return;
+  const int b = gptr[l], e = gptr[l + 1];
+  int sum = 0;
+  for (int i = b + lane; i < e; i += 32) {
+    const int g = gate[i], q1 = adj_ptr[g + 1];
+    int c = 0;
+    for (int q = adj_ptr[g]; q < q1; ++q) {
+      const int t = map[adj_idx[q]];
+      c += t >= b && t < e;
+    }
+    aend[i] = c;
+    sum += c;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  int base = 0;
+  if (lane == 0) base = (int)atomicAdd(total, (unsigned int)sum);
+  base = __shfl_sync(0xffffffffu, base, 0);
+  for (int i0 = b; i0 < e; i0 += 32) {
+    const int i = i0 + lane;
+    const int c = i < e ? aend[i] : 0;
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (i < e) {
+      int at = base + inc - c;
+      abeg[i] = at;
+      aend[i] = at + c;
+      const int g = gate[i], q1 = adj_ptr[g + 1];
+      for (int q = adj_ptr[g]; q < q1; ++q) {
+        const int t = map[adj_idx[q]];
+        if (t >= b && t < e) aidx[at++] = (int16_t)(t - b);
+      }
+    }
+    base += __shfl_sync(0xffffffffu, inc, 31);
+  }
+}
+
+// In-leaf adjacency on the host, for batches that list a gate more than once.
 struct LeafHost {
   std::vector<int32_t> aptr;
   std::vector<int16_t> aidx;
-  std::vector<int32_t> order;
 };
 
 // In-leaf adjacency of leaves [l0, l1) into aptr (counts relative to the
@@ -567,11 +644,6 @@ static void leaf_adjacency(const fx_design *d, int l0, int l1, const int32_t *le
 static int build_leaf_host(const fx_design *d, int L, const int32_t *leaf_ptr,
                            const int32_t *leaf_gate, LeafHost &h) {
   const int32_t G = leaf_ptr[L];
-  for (int l = 0; l < L; ++l)
-    if (leaf_ptr[l + 1] - leaf_ptr[l] > kLeafMax) {
-      set_error("leaf %d has %d gates (limit %d)", l, leaf_ptr[l + 1] - leaf_ptr[l], kLeafMax);
-      return FX_EINVAL;
-    }
   for (int32_t i = 0; i < G; ++i)
     if (leaf_gate[i] < 0 || leaf_gate[i] >= d->n) {
       set_error("leaf gate %d out of range", leaf_gate[i]);
@@ -618,11 +690,6 @@ static int build_leaf_host(const fx_design *d, int L, const int32_t *leaf_ptr,
     h.aidx.reserve(off);
     for (auto &p : part) h.aidx.insert(h.aidx.end(), p.begin(), p.end());
   }
-  h.order.resize(L);
-  std::iota(h.order.begin(), h.order.end(), 0);
-  std::stable_sort(h.order.begin(), h.order.end(), [&](int a, int c) {
-    return leaf_ptr[a + 1] - leaf_ptr[a] > leaf_ptr[c + 1] - leaf_ptr[c];
-  });
   return FX_OK;
 }
 
@@ -719,57 +786,87 @@ extern "C" int fx_hapr_place_leaves(fx_ctx *ctx, fx_design *d, int32_t n_leaves,
   FX_CHECK_CUDA(cudaSetDevice(ctx->device));
   AllocScope alloc_scope(ctx->stream);
   cudaStream_t s = ctx->stream;
-  LeafHost h;
-  FX_TRY(build_leaf_host(d, n_leaves, leaf_ptr, leaf_gate, h));
+  for (int l = 0; l < n_leaves; ++l)
+    if (leaf_ptr[l + 1] - leaf_ptr[l] > kLeafMax) {
+      set_error("leaf %d has %d gates (limit %d)", l, leaf_ptr[l + 1] - leaf_ptr[l], kLeafMax);
+      return FX_EINVAL;
+    }
   const int32_t G = leaf_ptr[n_leaves];
-  const PairPlan plan = pair_plan(n_leaves, leaf_ptr, h.order);
-  DevBuf<int32_t> gptr, gate, aptr, order;
+  const std::vector<int32_t> host_order = leaf_order(n_leaves, leaf_ptr);
+  const PairPlan plan = pair_plan(n_leaves, leaf_ptr, host_order);
+  DevBuf<int32_t> gptr, gate, abeg, aend, order, map;
   DevBuf<int16_t> aidx;
   DevBuf<float4> reg;
   DevBuf<float> ox, oy;
   DevBuf<unsigned int> counter;
   FX_TRY(gptr.alloc((size_t)n_leaves + 1));
   FX_TRY(gate.alloc(G > 0 ? (size_t)G : 1));
-  FX_TRY(aptr.alloc((size_t)G + 1));
-  FX_TRY(aidx.alloc(h.aidx.empty() ? 1 : h.aidx.size()));
+  FX_TRY(abeg.alloc((size_t)G + 1));
+  FX_TRY(aend.alloc(G > 0 ? (size_t)G : 1));
   FX_TRY(order.alloc((size_t)n_leaves));
   FX_TRY(reg.alloc((size_t)n_leaves));
   FX_TRY(ox.alloc((size_t)d->n));
   FX_TRY(oy.alloc((size_t)d->n));
-  FX_TRY(counter.alloc(2));
+  FX_TRY(counter.alloc(4));
+  FX_TRY(map.alloc((size_t)d->n));
   auto up = [&](void *dst, const void *src, size_t bytes) {
     return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
   };
   FX_CHECK_CUDA(up(gptr.p, leaf_ptr, ((size_t)n_leaves + 1) * 4));
-  // The reference writes the positions slot by slot, leaf by leaf, so a gate
-  // listed more than once keeps its last slot's position. The kernels write
-  // concurrently: every slot but a gate's last goes up as ~gate and skips
-  // the write. Batches without repeats go up unchanged.
-  std::vector<int32_t> gate_last;
-  {
+  FX_CHECK_CUDA(up(gate.p, leaf_gate, (size_t)G * 4));
+  FX_CHECK_CUDA(up(order.p, host_order.data(), host_order.size() * 4));
+  FX_CHECK_CUDA(up(reg.p, region, (size_t)n_leaves * 16));
+  // slots of the gates, and whether each is listed once and in range
+  unsigned int flag = 0;
+  FX_CHECK_CUDA(cudaMemsetAsync(map.p, 0xff, (size_t)d->n * 4, s));
+  FX_CHECK_CUDA(cudaMemsetAsync(counter.p, 0, 16, s));
+  if (G > 0) {
+    leaf_map_kernel<<<(G + 255) / 256, 256, 0, s>>>(gate.p, G, d->n, map.p, counter.p + 2);
+    FX_CHECK_LAUNCH();
+    ctx->launches += 1;
+    FX_CHECK_CUDA(cudaMemcpyAsync(&flag, counter.p + 2, 4, cudaMemcpyDeviceToHost, s));
+    FX_CHECK_CUDA(cudaStreamSynchronize(s));
+  }
+  const int32_t *row_end = aend.p;
+  if (flag == 0) {
+    FX_TRY(aidx.alloc(d->a > 0 ? (size_t)d->a : 1));
+    leaf_adj_kernel<<<(n_leaves + 7) / 8, 256, 0, s>>>(n_leaves, gptr.p, gate.p, map.p,
+                                                       d->adj_ptr.p, d->adj_idx.p, counter.p + 3,
+                                                       abeg.p, aend.p, aidx.p);
+    FX_CHECK_LAUNCH();
+    ctx->launches += 1;
+  } else {
+    LeafHost h;
+    FX_TRY(build_leaf_host(d, n_leaves, leaf_ptr, leaf_gate, h));
+    // The reference writes the positions slot by slot, leaf by leaf, so a gate
+    // listed more than once keeps its last slot's position. The kernels write
+    // concurrently: every slot but a gate's last goes up as ~gate and skips
+    // the write.
+    std::vector<int32_t> gate_last(leaf_gate, leaf_gate + G);
     std::vector<uint8_t> seen((size_t)d->n, 0);
     for (int32_t i = G - 1; i >= 0; --i) {
       const int32_t g = leaf_gate[i];
-      if (seen[g]) {
-        if (gate_last.empty()) gate_last.assign(leaf_gate, leaf_gate + G);
-        gate_last[i] = ~g;
-      }
+      if (seen[g]) gate_last[i] = ~g;
       seen[g] = 1;
     }
+    FX_TRY(aidx.alloc(h.aidx.empty() ? 1 : h.aidx.size()));
+    FX_CHECK_CUDA(up(gate.p, gate_last.data(), (size_t)G * 4));
+    FX_CHECK_CUDA(up(abeg.p, h.aptr.data(), h.aptr.size() * 4));
+    FX_CHECK_CUDA(up(aidx.p, h.aidx.data(), h.aidx.size() * 2));
+    FX_CHECK_CUDA(cudaStreamSynchronize(s));  // gate_last and h go out of scope
+    row_end = abeg.p + 1;
   }
-  FX_CHECK_CUDA(up(gate.p, gate_last.empty() ? leaf_gate : gate_last.data(), (size_t)G * 4));
-  FX_CHECK_CUDA(up(aptr.p, h.aptr.data(), h.aptr.size() * 4));
-  FX_CHECK_CUDA(up(aidx.p, h.aidx.data(), h.aidx.size() * 2));
-  FX_CHECK_CUDA(up(order.p, h.order.data(), h.order.size() * 4));
-  FX_CHECK_CUDA(up(reg.p, region, (size_t)n_leaves * 16));
-  FX_CHECK_CUDA(up(ox.p, out_x, (size_t)d->n * 4));
-  FX_CHECK_CUDA(up(oy.p, out_y, (size_t)d->n * 4));
+  // gates outside the batch keep the caller's positions
+  if (flag != 0 || G != d->n) {
+    FX_CHECK_CUDA(up(ox.p, out_x, (size_t)d->n * 4));
+    FX_CHECK_CUDA(up(oy.p, out_y, (size_t)d->n * 4));
+  }
   if (d->trace_on) {
     FX_TRY(d->leaf_trace.alloc(G > 0 ? (size_t)G : 1));
     FX_CHECK_CUDA(cudaMemsetAsync(d->leaf_trace.p, 0, (size_t)std::max(G, 1) * 8, s));
     d->leaf_trace_n = G;
   }
-  LeafBatch b{gptr.p, gate.p, aptr.p, aidx.p, reg.p, order.p, n_leaves,
+  LeafBatch b{gptr.p, gate.p, abeg.p, row_end, aidx.p, reg.p, order.p, n_leaves,
               cfg->force_iterations, cfg->attract_weight, cfg->repel_weight,
               cfg->damping, cfg->dt, ox.p, oy.p, counter.p,
               d->trace_on ? d->leaf_trace.p : nullptr};
@@ -835,7 +932,7 @@ extern "C" int fx_hapr_place_leaves(fx_ctx *ctx, fx_design *d, int32_t n_leaves,
   FX_CHECK_CUDA(cudaMemcpyAsync(out_y, oy.p, (size_t)d->n * 4, cudaMemcpyDeviceToHost, s));
   FX_CHECK_CUDA(cudaStreamSynchronize(s));
   if (out_schedule) *out_schedule = schedule;
-  for (auto *p : {&gptr, &gate, &aptr, &order}) p->release();
+  for (auto *p : {&gptr, &gate, &abeg, &aend, &order, &map}) p->release();
   aidx.release();
   reg.release();
   ox.release();
