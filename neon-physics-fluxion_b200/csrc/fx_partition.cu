@@ -286,9 +286,35 @@ __global__ void part_div_kernel(int n, const int32_t *__restrict__ clp,
   v[p] = r > 0.f ? __fdiv_rn(y, r) : y;
 }
 
-// FX_PART_FP64: one warp per chunk (<= kPartChunk positions of one cluster)
-// sums x, x^2 and v.x in FP64; one thread per cluster then adds its chunks
-// in order, so the reductions are deterministic.
+// FX_PART_FP64 sums of a cluster: s1 = sum x, s2 = sum x^2, s3 = sum v.x over
+// chunks of kPartChunk positions, each chunk by 32 strided sequential sums and
+// a shuffle tree, chunks added in order; every kernel below keeps this order.
+__device__ __forceinline__ double tree_sum(double s) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// Mean and norm of a cluster of n positions (|x - mean|^2 = sum(x^2) - n
+// mean^2: 1^T L v = 0, so no cancellation); without `deflate` (the start
+// vector) the norm only. nrm 0 where it is too small to divide by.
+__device__ __forceinline__ void mean_norm(double s1, double s2, double n, int deflate,
+                                          float &mean, float &nrm) {
+  const double m = deflate ? s1 / n : 0.0;
+  const double var = deflate ? fmax(s2 - s1 * m, 0.0) : s2;
+  const double norm = sqrt(var);
+  mean = (float)m;
+  nrm = norm > 1e-10 ? (float)norm : 0.f;
+}
+
+__device__ __forceinline__ float normed(float x, float mean, float nrm) {
+  const float y = __fsub_rn(x, mean);
+  return nrm > 0.f ? __fdiv_rn(y, nrm) : y;
+}
+
+// One warp per chunk (<= kPartChunk positions of one cluster) sums x, x^2
+// and v.x in FP64; one thread per cluster then adds its chunks in order, so
+// the reductions are deterministic.
 __global__ void part_chunk_kernel(int K, const int32_t *__restrict__ ck_beg,
                                   const int32_t *__restrict__ ck_end,
                                   const int32_t *__restrict__ ck_cl,
@@ -298,18 +324,28 @@ __global__ void part_chunk_kernel(int K, const int32_t *__restrict__ ck_beg,
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= K || !active[ck_cl[k]]) return;
   double s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  for (int p = ck_beg[k] + lane; p < ck_end[k]; p += 32) {
-    const double a = (double)x[p];
-    s1 += a;
-    s2 += a * a;
-    if (v) s3 += (double)v[p] * a;
-  }
+  // eight loads in flight per lane, added in order
+  const int e = ck_end[k];
+  for (int p0 = ck_beg[k] + lane; p0 < e; p0 += 32 * 8) {
+    float a8[8], v8[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s1 += __shfl_down_sync(0xffffffffu, s1, o);
-    s2 += __shfl_down_sync(0xffffffffu, s2, o);
-    s3 += __shfl_down_sync(0xffffffffu, s3, o);
+    for (int r = 0; r < 8; ++r) {
+      const int p = p0 + 32 * r;
+      a8[r] = p < e ? x[p] : 0.f;
+      v8[r] = v && p < e ? v[p] : 0.f;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (p0 + 32 * r >= e) break;
+      const double a = (double)a8[r];
+      s1 += a;
+      s2 += a * a;
+      if (v) s3 += (double)v8[r] * a;
+    }
   }
+  s1 = tree_sum(s1);
+  s2 = tree_sum(s2);
+  s3 = tree_sum(s3);
   if (lane == 0) {
     part[3 * k] = s1;
     part[3 * k + 1] = s2;
@@ -317,9 +353,8 @@ __global__ void part_chunk_kernel(int K, const int32_t *__restrict__ ck_beg,
   }
 }
 
-// Mean and norm per cluster (|x - mean|^2 = sum(x^2) - n mean^2: 1^T L v = 0,
-// so no cancellation), the Rayleigh quotient v.Lv of the unit v, and the
-// stop test. Without `deflate` (the start vector): norm only.
+// Mean and norm per cluster, the Rayleigh quotient v.Lv of the unit v, and
+// the stop test.
 __global__ void part_combine_kernel(int C, const int32_t *__restrict__ beg,
                                     const int32_t *__restrict__ end,
                                     const int32_t *__restrict__ cl_ck,
@@ -336,18 +371,276 @@ __global__ void part_combine_kernel(int C, const int32_t *__restrict__ beg,
     s2 += part[3 * k + 1];
     s3 += part[3 * k + 2];
   }
-  const double n = (double)(end[c] - beg[c]);
-  const double m = deflate ? s1 / n : 0.0;
-  const double var = deflate ? fmax(s2 - s1 * m, 0.0) : s2;
-  const double norm = sqrt(var);
-  mean[c] = (float)m;
-  nrm[c] = norm > 1e-10 ? (float)norm : 0.f;
+  mean_norm(s1, s2, (double)(end[c] - beg[c]), deflate, mean[c], nrm[c]);
   if (!deflate) return;
   const double prev = lambda[c];
   lambda[c] = s3;
   iters[c] += 1;
   if (tol > 0.0 && iters[c] > 1 && fabs(s3 - prev) <= tol * fabs(s3))
     active[c] = 2;  // converged: this update is the last
+}
+
+// ---- fixed iteration counts on clusters of several chunks --------------------
+// Two launches an iteration instead of four: the chunk sums with the
+// per-cluster combination in the last block to finish, and a product that
+// normalises its inputs as it reads them (v_j = (x_j - mean) / norm, a
+// division per neighbour, but no pass of its own over the vector). 22 us an
+// iteration at 100k gates against 37 (ncu cold); bound by the latency of the
+// sums' chain and of the gathers.
+constexpr int kSumThreads = 512;
+
+__global__ void __launch_bounds__(kSumThreads)
+part_sums_kernel(int C, const int32_t *__restrict__ ck_beg, const int32_t *__restrict__ ck_end,
+                 const int32_t *__restrict__ cl_ck, const int32_t *__restrict__ beg,
+                 const int32_t *__restrict__ end, const float *__restrict__ x, int deflate,
+                 double *__restrict__ part, unsigned int *__restrict__ done,
+                 float *__restrict__ mean, float *__restrict__ nrm) {
+  // the block brings its chunk to shared memory in one round of loads; then
+  // warp 0 sums x and warp 1 x^2 (a lane's 128 sums are a chain)
+  __shared__ float buf[kPartChunk];
+  const int k = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = ck_beg[k], n = ck_end[k] - b;
+  float v[kPartChunk / kSumThreads];
+#pragma unroll
+  for (int r = 0; r < kPartChunk / kSumThreads; ++r) {
+    const int i = r * kSumThreads + threadIdx.x;
+    v[r] = i < n ? x[b + i] : 0.f;
+  }
+#pragma unroll
+  for (int r = 0; r < kPartChunk / kSumThreads; ++r) buf[r * kSumThreads + threadIdx.x] = v[r];
+  __syncthreads();
+  if (w < 2) {
+    double s = 0.0;
+    if (w == 0) {
+#pragma unroll 8
+      for (int i = lane; i < n; i += 32) s += (double)buf[i];
+    } else {
+#pragma unroll 8
+      for (int i = lane; i < n; i += 32) {
+        const double a = (double)buf[i];
+        s += a * a;
+      }
+    }
+    s = tree_sum(s);
+    if (lane == 0) part[3 * k + w] = s;
+  }
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int c = threadIdx.x; c < C; c += blockDim.x) {
+    double s1 = 0.0, s2 = 0.0;
+    for (int q = cl_ck[c]; q < cl_ck[c + 1]; ++q) {
+      s1 += __ldcg(part + 3 * q);
+      s2 += __ldcg(part + 3 * q + 1);
+    }
+    mean_norm(s1, s2, (double)(end[c] - beg[c]), deflate, mean[c], nrm[c]);
+  }
+  if (threadIdx.x == 0) *done = 0u;
+}
+
+// v = normed(x) and lv = L v, in the order of part_spmv_csr_kernel.
+__global__ void part_step_kernel(int n, const int32_t *__restrict__ rp,
+                                 const int32_t *__restrict__ col,
+                                 const int32_t *__restrict__ clp,
+                                 const float *__restrict__ deg, const float *__restrict__ mean,
+                                 const float *__restrict__ nrm, const float *__restrict__ x,
+                                 float *__restrict__ v, float *__restrict__ lv) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int c = clp[p];
+  if (c < 0) return;
+  const float m = mean[c], r = nrm[c];
+  const float vp = normed(x[p], m, r);
+  v[p] = vp;
+  float l = __fmul_rn(deg[p], vp);
+  const int e1 = rp[p + 1];
+  // eight neighbours' loads and divisions in flight, subtracted in order
+  for (int e = rp[p]; e < e1; e += 8) {
+    int j[8];
+    float y[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) j[q] = e + q < e1 ? col[e + q] : p;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) y[q] = x[j[q]];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) y[q] = normed(y[q], m, r);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (e + q < e1) l = __fsub_rn(l, y[q]);
+  }
+  lv[p] = l;
+}
+
+// ---- a whole depth of clusters of one chunk each --------------------------------
+// A block per cluster of at most kPartChunk positions does all that the depth
+// does to it: the in-cluster CSR, every power iteration with the vectors in
+// shared memory, the stable sort by Fiedler value (position breaks ties, so
+// a bitonic sort of (key, place) pairs is stable) and the new order. One
+// launch of 141 us (a depth of 100k gates, ncu cold) instead of 4 * 30 + 25
+// launches of 1.2 ms: the lower depths' clusters of some hundred gates left
+// each launch waiting on one chain of sums. Bound by that chain (a lane's 128
+// dependent FP64 sums) and the barriers of 30 iterations. The sums keep the
+// chunked kernels' order, so the orders that come out are the same.
+// In its own segment a block overwrites perm and pos_of; other blocks only ask
+// whether a gate's place lies in their own segment, which no write changes.
+__host__ __device__ inline int pow2_above(int n) {
+  int p = 32;
+  while (p < n) p <<= 1;
+  return p;
+}
+static size_t part_small_smem(int most) {
+  return (size_t)pow2_above(most) * 8 + (size_t)most * 8 + ((size_t)most + 1) * 4;
+}
+
+__global__ void __launch_bounds__(1024)
+part_small_kernel(const int32_t *__restrict__ beg, const int32_t *__restrict__ end, int most,
+                  const int32_t *__restrict__ adj_ptr, const int32_t *__restrict__ adj_idx,
+                  const float *__restrict__ sin_tab, int iterations, double tol,
+                  int32_t *perm, int32_t *pos_of, uint16_t *__restrict__ col,
+                  unsigned int *__restrict__ total, unsigned long long *__restrict__ iters) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  uint64_t *key = reinterpret_cast<uint64_t *>(raw);
+  float *v = reinterpret_cast<float *>(key + pow2_above(most));
+  float *lv = v + most;
+  int32_t *rp = reinterpret_cast<int32_t *>(lv + most);
+  __shared__ int32_t wsum[32];
+  __shared__ unsigned int base_sh;
+  __shared__ double sums[3];
+  const int T = blockDim.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int b = beg[blockIdx.x], e = end[blockIdx.x], n = e - b;
+  // in-cluster CSR: counts, row starts, columns (local places)
+  for (int i = t; i < n; i += T) {
+    const int g = perm[b + i], q1 = adj_ptr[g + 1];
+    int c = 0;
+    for (int q = adj_ptr[g]; q < q1; ++q) c += (unsigned)(pos_of[adj_idx[q]] - b) < (unsigned)n;
+    rp[i + 1] = c;
+  }
+  __syncthreads();
+  const int per = (n + T - 1) / T, i0 = min(n, t * per), i1 = min(n, i0 + per);
+  int run = 0;
+  for (int i = i0; i < i1; ++i) run += rp[i + 1];
+  int inc = run;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) wsum[w] = inc;
+  __syncthreads();
+  int at = inc - run;
+  for (int q = 0; q < w; ++q) at += wsum[q];
+  for (int i = i0; i < i1; ++i) {
+    at += rp[i + 1];
+    rp[i + 1] = at;
+  }
+  if (t == 0) rp[0] = 0;
+  __syncthreads();
+  if (t == 0) base_sh = atomicAdd(total, (unsigned int)rp[n]);
+  __syncthreads();
+  uint16_t *mine = col + base_sh;
+  for (int i = t; i < n; i += T) {
+    const int g = perm[b + i], q1 = adj_ptr[g + 1];
+    int k = rp[i];
+    for (int q = adj_ptr[g]; q < q1; ++q) {
+      const int r = pos_of[adj_idx[q]] - b;
+      if ((unsigned)r < (unsigned)n) mine[k++] = (uint16_t)r;
+    }
+    lv[i] = sin_tab[i];
+  }
+  __syncthreads();
+  // sums over x = lv (and v), one kind per warp; then v = normed(lv)
+  auto reduce = [&](bool with_v) {
+    if (w < 2 || (w == 2 && with_v)) {
+      double s = 0.0;
+      if (w == 0) {
+#pragma unroll 8
+        for (int i = lane; i < n; i += 32) s += (double)lv[i];
+      } else if (w == 1) {
+#pragma unroll 8
+        for (int i = lane; i < n; i += 32) {
+          const double a = (double)lv[i];
+          s += a * a;
+        }
+      } else {
+#pragma unroll 8
+        for (int i = lane; i < n; i += 32) s += (double)v[i] * (double)lv[i];
+      }
+      s = tree_sum(s);
+      if (lane == 0) sums[w] = 0.0 + s;
+    }
+    __syncthreads();
+  };
+  auto normalise = [&](int deflate) {
+    float m, r;
+    mean_norm(sums[0], sums[1], (double)n, deflate, m, r);
+    for (int i = t; i < n; i += T) v[i] = normed(lv[i], m, r);
+    __syncthreads();
+  };
+  reduce(false);
+  normalise(0);
+  double lambda = 0.0;
+  int it = 0;
+  while (it < iterations) {
+    for (int i = t; i < n; i += T) {
+      const int k1 = rp[i + 1], k0 = rp[i];
+      float l = __fmul_rn((float)(k1 - k0), v[i]);
+      for (int k = k0; k < k1; k += 8) {
+        int j[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) j[q] = k + q < k1 ? mine[k + q] : i;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (k + q < k1) l = __fsub_rn(l, v[j[q]]);
+      }
+      lv[i] = l;
+    }
+    __syncthreads();
+    reduce(true);
+    ++it;
+    const double prev = lambda;
+    lambda = sums[2];
+    const bool stop = tol > 0.0 && it > 1 && fabs(lambda - prev) <= tol * fabs(lambda);
+    normalise(1);  // a converged cluster takes this update as its last
+    if (stop) break;
+  }
+  if (t == 0 && it > 0) atomicAdd(iters, (unsigned long long)it);
+  // stable sort by value (-0.0 as +0.0), then the new order
+  const int P = pow2_above(n);
+  for (int i = t; i < P; i += T) {
+    uint64_t k = ~0ull;
+    if (i < n) {
+      float f = v[i];
+      if (f == 0.f) f = 0.f;
+      const uint32_t u = __float_as_uint(f);
+      k = (uint64_t)((u & 0x80000000u) ? ~u : (u | 0x80000000u)) << 32 | (uint32_t)i;
+    }
+    key[i] = k;
+  }
+  __syncthreads();
+  for (int size = 2; size <= P; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int j = t; j < P / 2; j += T) {
+        const int lo = 2 * j - (j & (stride - 1)), hi = lo + stride;
+        const uint64_t x = key[lo], y = key[hi];
+        if ((x > y) == ((lo & size) == 0)) {
+          key[lo] = y;
+          key[hi] = x;
+        }
+      }
+      __syncthreads();
+    }
+  int32_t *gate = reinterpret_cast<int32_t *>(lv);
+  for (int i = t; i < n; i += T) gate[i] = perm[b + i];
+  __syncthreads();
+  for (int i = t; i < n; i += T) {
+    const int g = gate[(uint32_t)key[i]];
+    perm[b + i] = g;
+    pos_of[g] = b + i;
+  }
 }
 
 __global__ void part_retire_kernel(int C, int32_t *__restrict__ active,
@@ -538,6 +831,13 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
     DevBuf<double> part, lambda;
     DevBuf<uint32_t> keys[2], th, ts, dt;
     DevBuf<int32_t> vals[2], slot_pos;
+    DevBuf<float> lv2;
+    DevBuf<unsigned int> counters;         // last-block counter, CSR entries
+    DevBuf<unsigned long long> small_its;  // iterations of the one-chunk depths
+    FX_TRY(counters.alloc(2));
+    FX_TRY(small_its.alloc(1));
+    FX_CHECK_CUDA(cudaMemsetAsync(counters.p, 0, 8, s));
+    FX_CHECK_CUDA(cudaMemsetAsync(small_its.p, 0, 8, s));
     FX_TRY(upload(d_sin, sin_tab, s));
     FX_TRY(clp.alloc(N));
     FX_TRY(clg.alloc(N));
@@ -576,6 +876,23 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       if (C == 0) continue;
       FX_TRY(upload(beg, hb, s));
       FX_TRY(upload(end, he, s));
+      int32_t most = 0;
+      for (int c = 0; c < C; ++c) most = std::max(most, he[c] - hb[c]);
+      if (!exact && most <= kPartChunk) {
+        // one block per cluster; two to four positions a thread
+        const size_t smem = part_small_smem(most);
+        const int threads = std::min(1024, std::max(96, (most / 2 + 31) / 32 * 32));
+        FX_TRY(raise_smem_limit((const void *)part_small_kernel, (int)smem));
+        FX_CHECK_CUDA(cudaMemsetAsync(counters.p + 1, 0, 4, s));
+        part_small_kernel<<<C, threads, smem, s>>>(
+            beg.p, end.p, most, d->adj_ptr.p, d->adj_idx.p, d_sin.p, cfg->power_iterations,
+            cfg->tol, perm[cur].p, pos_of.p, reinterpret_cast<uint16_t *>(col.p),
+            counters.p + 1, small_its.p);
+        FX_CHECK_LAUNCH();
+        ctx->launches += 1;
+        FX_CHECK_CUDA(cudaStreamSynchronize(s));  // beg and end are reused
+        continue;
+      }
       FX_TRY(upload(off, hoff, s));
       FX_TRY(upload(act, std::vector<int32_t>((size_t)C, 1), s));
       FX_TRY(mean.alloc(C));
@@ -612,8 +929,31 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       part_csr_kernel<<<nb, 256, 0, s>>>(N, perm[cur].p, pos_of.p, d->adj_ptr.p, d->adj_idx.p,
                                          clp.p, clg.p, rp.p, col.p);
       ctx->launches += 4;
+      const bool fixed = !exact && cfg->tol <= 0.0;
+      if (fixed) {
+        // v holds the start vector; iterate x -> v = normed(x), lv = L v
+        FX_TRY(lv2.alloc(N));
+        float *x = lv2.p, *y = lv.p;
+        FX_CHECK_CUDA(cudaMemcpyAsync(x, v.p, (size_t)N * 4, cudaMemcpyDeviceToDevice, s));
+        auto sums = [&](int deflate) {
+          part_sums_kernel<<<K, kSumThreads, 0, s>>>(C, ck_beg.p, ck_end.p, cl_ck.p, beg.p, end.p, x,
+                                            deflate, part.p, counters.p, mean.p, nrm.p);
+        };
+        sums(0);
+        for (int it = 0; it < cfg->power_iterations; ++it) {
+          part_step_kernel<<<nb, 256, 0, s>>>(N, rp.p, col.p, clp.p, deg.p, mean.p, nrm.p, x, v.p,
+                                              y);
+          std::swap(x, y);
+          sums(1);
+        }
+        part_div_kernel<<<nb, 256, 0, s>>>(N, clp.p, act.p, x, mean.p, nrm.p, v.p);
+        FX_CHECK_LAUNCH();
+        ctx->launches += 2 + 2 * cfg->power_iterations;
+        total_iters += (int64_t)cfg->power_iterations * C;
+      }
       // normalise the start vector (:151-156)
-      if (exact) {
+      if (fixed) {
+      } else if (exact) {
         part_seq_kernel<<<C, 32, 0, s>>>(C, beg.p, end.p, v.p, 0, nrm.p);
       } else {
         part_chunk_kernel<<<kb, 256, 0, s>>>(K, ck_beg.p, ck_end.p, ck_cl.p, act.p, v.p,
@@ -621,11 +961,13 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
         part_combine_kernel<<<cb, 64, 0, s>>>(C, beg.p, end.p, cl_ck.p, part.p, 0, 0.0, act.p,
                                               mean.p, nrm.p, lambda.p, iters.p);
       }
-      part_div_kernel<<<nb, 256, 0, s>>>(N, clp.p, act.p, v.p, nullptr, nrm.p, v.p);
-      FX_CHECK_LAUNCH();
-      ctx->launches += exact ? 4 : 5;
+      if (!fixed) {
+        part_div_kernel<<<nb, 256, 0, s>>>(N, clp.p, act.p, v.p, nullptr, nrm.p, v.p);
+        FX_CHECK_LAUNCH();
+        ctx->launches += exact ? 4 : 5;
+      }
       int it = 0;
-      while (it < cfg->power_iterations) {
+      while (!fixed && it < cfg->power_iterations) {
         part_spmv_csr_kernel<<<nb, 256, 0, s>>>(N, rp.p, col.p, clp.p, act.p, deg.p, v.p,
                                                 lv.p);
         ++it;
@@ -658,7 +1000,7 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       }
       if (exact) {
         total_iters += (int64_t)it * C;
-      } else {
+      } else if (!fixed) {
         std::vector<int32_t> hit((size_t)C);
         FX_CHECK_CUDA(cudaMemcpyAsync(hit.data(), iters.p, (size_t)C * 4,
                                       cudaMemcpyDeviceToHost, s));
@@ -690,6 +1032,10 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       cur ^= 1;
       FX_CHECK_CUDA(cudaStreamSynchronize(s));
     }
+    unsigned long long si = 0;
+    FX_CHECK_CUDA(cudaMemcpyAsync(&si, small_its.p, 8, cudaMemcpyDeviceToHost, s));
+    FX_CHECK_CUDA(cudaStreamSynchronize(s));
+    total_iters += (int64_t)si;
   }
   // outputs: leaves in position order, with their regions
   if (!nodes.empty()) {
