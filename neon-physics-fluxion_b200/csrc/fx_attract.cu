@@ -80,12 +80,15 @@ __global__ void __launch_bounds__(kGates)
 attract_kernel(const int32_t *__restrict__ adj_ptr,
                const int32_t *__restrict__ adj_idx, const float *__restrict__ x,
                const float *__restrict__ y, int n, float k,
-               float2 *__restrict__ out) {
+               float *__restrict__ out) {
   const int g0 = blockIdx.x * kGates, g = g0 + threadIdx.x;
   const bool valid = g < n;
   const float xi = valid ? x[g] : 0.f, yi = valid ? y[g] : 0.f;
   const float2 f = spring_block(adj_ptr, adj_idx, x, y, n, g0, k, xi, yi);
-  if (valid) out[g] = f;
+  if (valid) {
+    out[g] = f.x;
+    out[n + g] = f.y;
+  }
 }
 
 struct StepArgs {
@@ -236,7 +239,7 @@ fused_step_kernel(StepArgs a) {
   }
 }
 
-int attraction_run(fx_ctx *ctx, fx_design *d, float k, float2 *out,
+int attraction_run(fx_ctx *ctx, fx_design *d, float k, float *out,
                    cudaStream_t s) {
   const int nb = (d->n + kGates - 1) / kGates;
   attract_kernel<<<nb, kGates, 0, s>>>(d->adj_ptr.p, d->adj_idx.p,
@@ -310,15 +313,12 @@ extern "C" int fx_stage_attraction(fx_ctx *ctx, fx_design *d, float k,
   FX_CHECK_CUDA(cudaSetDevice(ctx->device));
   AllocScope alloc_scope(ctx->stream);
   cudaStream_t s = ctx->stream;
-  FX_TRY(attraction_run(ctx, d, k, d->fattr.p, s));
-  std::vector<float2> f((size_t)d->n);
-  FX_CHECK_CUDA(cudaMemcpyAsync(f.data(), d->fattr.p, (size_t)d->n * 8,
-                                cudaMemcpyDeviceToHost, s));
+  float *f = reinterpret_cast<float *>(d->fattr.p);
+  const size_t n = (size_t)d->n;
+  FX_TRY(attraction_run(ctx, d, k, f, s));
+  if (out_fx) FX_CHECK_CUDA(cudaMemcpyAsync(out_fx, f, n * 4, cudaMemcpyDeviceToHost, s));
+  if (out_fy) FX_CHECK_CUDA(cudaMemcpyAsync(out_fy, f + n, n * 4, cudaMemcpyDeviceToHost, s));
   FX_CHECK_CUDA(cudaStreamSynchronize(s));
-  for (int i = 0; i < d->n; ++i) {
-    if (out_fx) out_fx[i] = f[i].x;
-    if (out_fy) out_fy[i] = f[i].y;
-  }
   return FX_OK;
 }
 

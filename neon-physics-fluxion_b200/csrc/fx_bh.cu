@@ -1620,6 +1620,22 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
 
 using namespace fx;
 
+namespace fx {
+// The stage call's outputs in the caller's layout: forces as two arrays, keys
+// in gate order (perm maps sorted position -> gate).
+__global__ void bh_unpack_kernel(int n, const float2 *__restrict__ force,
+                                 const uint32_t *__restrict__ skeys,
+                                 const int32_t *__restrict__ perm, float *__restrict__ fx,
+                                 float *__restrict__ fy, uint32_t *__restrict__ keys) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float2 f = force[i];
+  fx[i] = f.x;
+  fy[i] = f.y;
+  keys[perm[i]] = skeys[i];
+}
+}  // namespace fx
+
 extern "C" int fx_stage_barnes_hut_walk(fx_ctx *ctx, fx_design *d, float k, float theta,
                                         float min_dist, int32_t walk, float *out_fx,
                                         float *out_fy, uint32_t *out_keys, int32_t *out_perm,
@@ -1639,26 +1655,28 @@ extern "C" int fx_stage_barnes_hut_walk(fx_ctx *ctx, fx_design *d, float k, floa
   FX_TRY(bh_run(ctx, d, k, theta, min_dist, walk, s, out_terms ? terms.p : nullptr));
   if (out_terms)
     FX_CHECK_CUDA(cudaMemcpyAsync(out_terms, terms.p, n * 4, cudaMemcpyDeviceToHost, s));
-  std::vector<float2> f(n);
-  std::vector<uint32_t> skeys(n);
-  std::vector<int32_t> perm(n);
+  // straight into the caller's arrays (unpacking on the host took 1.1 of 1.7 ms
+  // at 300k points); the scratch is the stage's own force buffer and the sort's
+  // second key buffer
+  float *ux = reinterpret_cast<float *>(d->fattr.p), *uy = ux + n;
+  uint32_t *uk = d->bh.keys[1].p;
+  bh_unpack_kernel<<<((int)n + 255) / 256, 256, 0, s>>>((int)n, d->bh.force.p, d->bh.keys[0].p,
+                                                        d->bh.idx[0].p, ux, uy, uk);
+  FX_CHECK_LAUNCH();
+  ctx->launches += 1;
   unsigned int err = 0;
-  FX_CHECK_CUDA(cudaMemcpyAsync(f.data(), d->bh.force.p, n * 8, cudaMemcpyDeviceToHost, s));
-  FX_CHECK_CUDA(cudaMemcpyAsync(skeys.data(), d->bh.keys[0].p, n * 4, cudaMemcpyDeviceToHost, s));
-  FX_CHECK_CUDA(cudaMemcpyAsync(perm.data(), d->bh.idx[0].p, n * 4, cudaMemcpyDeviceToHost, s));
+  auto out = [&](void *dst, const void *src) {
+    return dst ? cudaMemcpyAsync(dst, src, n * 4, cudaMemcpyDeviceToHost, s) : cudaSuccess;
+  };
+  FX_CHECK_CUDA(out(out_fx, ux));
+  FX_CHECK_CUDA(out(out_fy, uy));
+  FX_CHECK_CUDA(out(out_keys, uk));
+  FX_CHECK_CUDA(out(out_perm, d->bh.idx[0].p));
   if (out_root)
     FX_CHECK_CUDA(cudaMemcpyAsync(out_root, d->bh.root.p, 12, cudaMemcpyDeviceToHost, s));
   FX_CHECK_CUDA(cudaMemcpyAsync(&err, d->bh.bbox.p + 4, 4, cudaMemcpyDeviceToHost, s));
   FX_CHECK_CUDA(cudaStreamSynchronize(s));
   FX_TRY(bh_error(err));
-  for (size_t i = 0; i < n; ++i) {
-    if (out_fx) out_fx[i] = f[i].x;
-    if (out_fy) out_fy[i] = f[i].y;
-  }
-  // keys in gate order; perm maps sorted position -> gate
-  if (out_keys)
-    for (size_t i = 0; i < n; ++i) out_keys[perm[i]] = skeys[i];
-  if (out_perm) std::copy(perm.begin(), perm.end(), out_perm);
   return FX_OK;
 }
 

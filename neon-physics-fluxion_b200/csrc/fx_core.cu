@@ -316,6 +316,7 @@ extern "C" int fx_ctx_destroy(fx_ctx *ctx) {
   cudaEventDestroy(ctx->join);
   if (ctx->tc_err) cudaFree(ctx->tc_err);
   if (ctx->readback) cudaFreeHost(ctx->readback);
+  ctx->sin_tab.release();
   cudaStreamDestroy(ctx->stream);
   cudaStreamDestroy(ctx->stream2);
   delete ctx;

@@ -128,7 +128,7 @@ __global__ void dens_gather_kernel(const float *__restrict__ x,
                                    const float *__restrict__ ex,
                                    const float *__restrict__ ey,
                                    const float *__restrict__ phi,
-                                   float2 *__restrict__ force,
+                                   float *__restrict__ fx, float *__restrict__ fy,
                                    double *__restrict__ partial,
                                    unsigned int *__restrict__ done,
                                    double *__restrict__ energy) {
@@ -138,8 +138,8 @@ __global__ void dens_gather_kernel(const float *__restrict__ x,
     const int c = bin_at(x[i], bw, G), r = bin_at(y[i], bh, G);
     const size_t b = (size_t)r * G + c;
     const float q = area[i];
-    force[i] = make_float2(__fmul_rn(__fmul_rn(q, ex[b]), weight),
-                           __fmul_rn(__fmul_rn(q, ey[b]), weight));
+    fx[i] = __fmul_rn(__fmul_rn(q, ex[b]), weight);
+    fy[i] = __fmul_rn(__fmul_rn(q, ey[b]), weight);
     e += 0.5 * (double)q * (double)phi[b];
   }
   last_block_sum(block_sum_double(e) * (double)weight, partial, done, energy);
@@ -195,7 +195,7 @@ static int dens_setup_fast(fx_design *d, int G, int precision, cudaStream_t s) {
   FX_TRY(w.ex.alloc(cells));
   FX_TRY(w.ey.alloc(cells));
   FX_TRY(w.energy.alloc(4096 + 8));
-  FX_TRY(w.force.alloc((size_t)d->n));
+  FX_TRY(w.force.alloc(2 * (size_t)d->n));
   const size_t g = (size_t)G;
   FX_CHECK_CUDA(cudaMemcpyAsync(w.tw.p, tw.data(), g * 16, cudaMemcpyHostToDevice, s));
   FX_CHECK_CUDA(cudaMemcpyAsync(w.qt.p, qt.data(), g * 16, cudaMemcpyHostToDevice, s));
@@ -234,7 +234,7 @@ static int dens_setup(fx_design *d, int G, int precision, cudaStream_t s) {
   FX_TRY(w.ex.alloc(cells));
   FX_TRY(w.ey.alloc(cells));
   FX_TRY(w.energy.alloc(4096 + 8));
-  FX_TRY(w.force.alloc((size_t)d->n));
+  FX_TRY(w.force.alloc(2 * (size_t)d->n));
   // The GEMMs are halved by the DCT's even/odd symmetry when G is a multiple
   // of 256 (tiles of 128 on each half). Not for 3xTF32: rows G-1-i come out
   // as E - O, and that difference magnifies the tensor cores' accumulation
@@ -501,7 +501,7 @@ int density_gather(fx_ctx *ctx, fx_design *d, const float *x, const float *y,
   if (nb > 4096) nb = 4096;
   dens_gather_kernel<<<nb, 256, 0, s>>>(x, y, d->area.p, d->n, G, bw, bh,
                                         weight, w.ex.p, w.ey.p, w.buf[3].p,
-                                        w.force.p, w.energy.p, (unsigned int *)(w.energy.p + 4096),
+                                        w.force.p, w.force.p + d->n, w.energy.p, (unsigned int *)(w.energy.p + 4096),
                                         w.energy.p + 4097);
   FX_CHECK_LAUNCH();
   ctx->launches += 1;
@@ -534,9 +534,9 @@ extern "C" int fx_stage_density(fx_ctx *ctx, fx_design *d, int32_t bins,
   FX_TRY(density_gather(ctx, d, x, y, bins, weight, s));
   DensityWork &w = d->dens;
   const size_t cells = (size_t)bins * bins, n = (size_t)d->n;
-  std::vector<float2> f(n);
   double e = 0.0;
-  FX_CHECK_CUDA(cudaMemcpyAsync(f.data(), w.force.p, n * 8, cudaMemcpyDeviceToHost, s));
+  if (out_fx) FX_CHECK_CUDA(cudaMemcpyAsync(out_fx, w.force.p, n * 4, cudaMemcpyDeviceToHost, s));
+  if (out_fy) FX_CHECK_CUDA(cudaMemcpyAsync(out_fy, w.force.p + n, n * 4, cudaMemcpyDeviceToHost, s));
   std::vector<float> rho_lo;
   if (out_rho) FX_CHECK_CUDA(cudaMemcpyAsync(out_rho, w.buf[0].p, cells * 4, cudaMemcpyDeviceToHost, s));
   if (out_rho && precision == FX_DCT_FP32) {
@@ -553,10 +553,6 @@ extern "C" int fx_stage_density(fx_ctx *ctx, fx_design *d, int32_t bins,
   if (tc_err) {
     set_error("tensor-core GEMM: a bounded wait expired (error word %u)", tc_err);
     return FX_ETIMEOUT;
-  }
-  for (size_t i = 0; i < n; ++i) {
-    if (out_fx) out_fx[i] = f[i].x;
-    if (out_fy) out_fy[i] = f[i].y;
   }
   for (size_t i = 0; i < rho_lo.size(); ++i) out_rho[i] += rho_lo[i];
   if (out_energy) *out_energy = e;

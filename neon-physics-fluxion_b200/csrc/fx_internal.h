@@ -179,7 +179,7 @@ struct DensityWork {
   DevBuf<uint16_t> bf[3];              // bf16 operand staging
   DevBuf<float> ex, ey;                // field
   DevBuf<double> energy;               // FP64 partials
-  DevBuf<float2> force;                // per gate
+  DevBuf<float> force;                 // per gate: x, then y (stage call)
   DevBuf<float> half_ws;               // half products before their placing
   // even/odd GEMMs (G a multiple of 256): the half operators
   // [C even rows | C odd rows], [C^T even cols | odd cols], Dx C^T, Dy C^T
@@ -274,6 +274,9 @@ struct fx_ctx {
   fx::StageTimer timer;
   int64_t launches = 0;
   cudaEvent_t marks[16] = {};
+  // sin(i * 2.71828), the power iteration's start vector: a table of the
+  // largest cluster seen (fx_partition.cu)
+  fx::DevBuf<float> sin_tab;
   int leaf_schedule = 0;           // last autotuned leaf schedule
   // FX_LEAF_AUTO decisions by batch shape (leaf count, mean leaf size and
   // iteration count, each as a power-of-two bucket)
@@ -302,7 +305,7 @@ struct fx_design {
   // clamps to the die); with the saved copy's flag.
   bool pos_in_box = false, saved_in_box = false;
   fx::DevBuf<unsigned int> box_flag;
-  fx::DevBuf<float2> fattr;      // attraction-only force output (stage API)
+  fx::DevBuf<float2> fattr;      // force outputs of the stage calls (n floats x, then n y)
   // force trace (fx_design_trace): each plain iteration stores its total
   // force, start positions and start velocities (6 x n floats)
   bool trace_on = false;
@@ -348,7 +351,7 @@ namespace fx {
 int congestion_alloc(fx_design *d, int cols, int rows, cudaStream_t s);
 int congestion_run(fx_ctx *ctx, fx_design *d, const float *dx, const float *dy,
                    int cols, int rows, cudaStream_t s);
-int attraction_run(fx_ctx *ctx, fx_design *d, float k, float2 *out, cudaStream_t s);
+int attraction_run(fx_ctx *ctx, fx_design *d, float k, float *out, cudaStream_t s);
 int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int walk,
            cudaStream_t s, int32_t *term_count = nullptr);
 int density_run(fx_ctx *ctx, fx_design *d, int G, float target, float weight,

@@ -823,10 +823,19 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
     FX_TRY(perm[1].alloc(N));
   }
   if (levels > 0) {
-    // the reference's start vector, from the host libm (as f32::sin)
-    std::vector<float> sin_tab((size_t)max_active);
-    for (int32_t i = 0; i < max_active; ++i) sin_tab[i] = std::sin((float)i * 2.71828f);
-    DevBuf<float> d_sin, deg, v, lv, mean, nrm;
+    // the reference's start vector, from the host libm (as f32::sin); the table
+    // depends on nothing else, so the context keeps the longest one made
+    DevBuf<float> &d_sin = ctx->sin_tab;
+    if (d_sin.n < (size_t)max_active) {
+      std::vector<float> sin_tab((size_t)max_active);
+      for (int32_t i = 0; i < max_active; ++i) sin_tab[i] = std::sin((float)i * 2.71828f);
+      if (upload(d_sin, sin_tab, s) != FX_OK || cudaStreamSynchronize(s) != cudaSuccess) {
+        d_sin.release();
+        set_error("fx_partition: start vector upload failed");
+        return FX_ECUDA;
+      }
+    }
+    DevBuf<float> deg, v, lv, mean, nrm;
     DevBuf<int32_t> clp, clg, beg, end, off, act, iters, any, ck_beg, ck_end, ck_cl, cl_ck;
     DevBuf<double> part, lambda;
     DevBuf<uint32_t> keys[2], th, ts, dt;
@@ -838,7 +847,6 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
     FX_TRY(small_its.alloc(1));
     FX_CHECK_CUDA(cudaMemsetAsync(counters.p, 0, 8, s));
     FX_CHECK_CUDA(cudaMemsetAsync(small_its.p, 0, 8, s));
-    FX_TRY(upload(d_sin, sin_tab, s));
     FX_TRY(clp.alloc(N));
     FX_TRY(clg.alloc(N));
     FX_TRY(deg.alloc(N));
