@@ -107,7 +107,6 @@ struct StepArgs {
   // bookkeeping for the next iteration
   unsigned int *bbox;          // box of the new positions (ordered ints) or null
   unsigned long long *dens_acc;  // density accumulator for the new positions
-  float4 *bbox_part;
   double *e_part;
   unsigned int *done;
   double *energy;
@@ -130,11 +129,28 @@ __device__ __forceinline__ float clampf_ref(float v, float lo, float hi) {
 
 // One gate per thread: F = attraction + Barnes-Hut + density (f32, in this
 // order), the damped step, then the new positions' density scatter and box.
+// Bound by L1 (neighbour gathers and the row sums' shared loads, 70 % of its
+// rate) and by the two barriers a chunk; 84 to 78 us at 1M gates since the box
+// is a reduction into memory instead of a last block's pass over all blocks'
+// boxes and the gate's own loads overlap the springs. Packed (x, y) positions,
+// half the gathers, were no faster (82 us) and cost a launch.
 __global__ void __launch_bounds__(kGates)
 fused_step_kernel(StepArgs a) {
   const int g0 = blockIdx.x * kGates, g = g0 + threadIdx.x;
   const bool valid = g < a.n;
+  // the gate's own inputs are loaded before the springs, whose chain of loads
+  // and sums they then overlap
   const float px = valid ? a.x[g] : 0.f, py = valid ? a.y[g] : 0.f;
+  const float vx0 = valid ? a.vx[g] : 0.f, vy0 = valid ? a.vy[g] : 0.f;
+  const float2 fb = valid && a.fbh ? a.fbh[g] : make_float2(0.f, 0.f);
+  const float q = valid && (a.ex || a.dens_acc) ? a.area[g] : 0.f;
+  float2 field = make_float2(0.f, 0.f);
+  size_t bi = 0;
+  if (valid && a.ex) {
+    const int c = bin_of(px, a.bw, a.G), r = bin_of(py, a.bh, a.G);
+    bi = (size_t)r * a.G + c;
+    field = make_float2(a.ex[bi], a.ey[bi]);
+  }
   const float2 s = spring_block(a.adj_ptr, a.adj_idx, a.x, a.y, a.n, g0, a.k, px, py);
   float nx = px, ny = py;
   double e_acc = 0.0;
@@ -143,19 +159,14 @@ fused_step_kernel(StepArgs a) {
   if (valid) {
     float fx = s.x, fy = s.y;
     if (a.fbh) {
-      const float2 b = a.fbh[g];
-      fx = __fadd_rn(fx, b.x);
-      fy = __fadd_rn(fy, b.y);
+      fx = __fadd_rn(fx, fb.x);
+      fy = __fadd_rn(fy, fb.y);
     }
     if (a.ex) {
-      const int c = bin_of(px, a.bw, a.G), r = bin_of(py, a.bh, a.G);
-      const size_t bi = (size_t)r * a.G + c;
-      const float q = a.area[g];
-      fx = __fadd_rn(fx, __fmul_rn(__fmul_rn(q, a.ex[bi]), a.dweight));
-      fy = __fadd_rn(fy, __fmul_rn(__fmul_rn(q, a.ey[bi]), a.dweight));
+      fx = __fadd_rn(fx, __fmul_rn(__fmul_rn(q, field.x), a.dweight));
+      fy = __fadd_rn(fy, __fmul_rn(__fmul_rn(q, field.y), a.dweight));
       if (a.phi) e_acc = 0.5 * (double)q * (double)a.phi[bi] * (double)a.dweight;
     }
-    const float vx0 = a.vx[g], vy0 = a.vy[g];
     if (a.trace) {
       const size_t n = (size_t)a.n;
       a.trace[g] = fx;
@@ -176,35 +187,48 @@ fused_step_kernel(StepArgs a) {
     if (a.dens_acc) {
       const int c = bin_of(nx, a.bw, a.G), r = bin_of(ny, a.bh, a.G);
       dbin = (long long)r * a.G + c;
-      dval = (unsigned long long)llrint((double)a.area[g] * 4294967296.0);
+      dval = (unsigned long long)llrint((double)q * 4294967296.0);
     }
   }
   if (a.dens_acc) agg_add_u64(a.dens_acc, dbin, dval);
-  // Box of the new positions and density energy: per-block values, then the
-  // last block combines them in block order.
+  // Box of the new positions: minima and maxima of ordered integers, exact in
+  // any order, straight into the box (re-armed by the tree build); a block
+  // only adds what the box does not cover yet.
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  float mnx = valid ? nx : FLT_MAX, mny = valid ? ny : FLT_MAX;
-  float mxx = valid ? nx : -FLT_MAX, mxy = valid ? ny : -FLT_MAX;
+  if (a.bbox) {
+    float mnx = valid ? nx : FLT_MAX, mny = valid ? ny : FLT_MAX;
+    float mxx = valid ? nx : -FLT_MAX, mxy = valid ? ny : -FLT_MAX;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-    mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-    mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-    mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+    for (int o = 16; o > 0; o >>= 1) {
+      mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
+      mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
+      mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
+      mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+    }
+    __shared__ float4 wbox[kGates / 32];
+    if (lane == 0) wbox[w] = make_float4(mnx, mny, mxx, mxy);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float4 bb = wbox[0];
+      for (int i = 1; i < kGates / 32; ++i) {
+        bb.x = fminf(bb.x, wbox[i].x);
+        bb.y = fminf(bb.y, wbox[i].y);
+        bb.z = fmaxf(bb.z, wbox[i].z);
+        bb.w = fmaxf(bb.w, wbox[i].w);
+      }
+      const uint4 cur = __ldcg(reinterpret_cast<const uint4 *>(a.bbox));
+      if (f2ord(bb.x) < cur.x) atomicMin(a.bbox + 0, f2ord(bb.x));
+      if (f2ord(bb.y) < cur.y) atomicMin(a.bbox + 1, f2ord(bb.y));
+      if (f2ord(bb.z) > cur.z) atomicMax(a.bbox + 2, f2ord(bb.z));
+      if (f2ord(bb.w) > cur.w) atomicMax(a.bbox + 3, f2ord(bb.w));
+    }
   }
-  __shared__ float4 wbox[kGates / 32];
-  if (lane == 0) wbox[w] = make_float4(mnx, mny, mxx, mxy);
+  // Density energy (a run's last step only): per-block sums, added by the
+  // last block in block order, sixteen loads in flight a thread.
+  if (!a.phi) return;
   const double esum = block_sum_double(e_acc);  // contains __syncthreads
   __shared__ bool last;
   if (threadIdx.x == 0) {
-    float4 bb = wbox[0];
-    for (int q = 1; q < kGates / 32; ++q) {
-      bb.x = fminf(bb.x, wbox[q].x);
-      bb.y = fminf(bb.y, wbox[q].y);
-      bb.z = fmaxf(bb.z, wbox[q].z);
-      bb.w = fmaxf(bb.w, wbox[q].w);
-    }
-    a.bbox_part[blockIdx.x] = bb;
     a.e_part[blockIdx.x] = esum;
     __threadfence();
     last = atomicAdd(a.done, 1u) == gridDim.x - 1;
@@ -212,29 +236,19 @@ fused_step_kernel(StepArgs a) {
   __syncthreads();
   if (!last) return;
   __threadfence();
-  float4 bb = make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX);
   double et = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kGates) {
-    const float4 q = __ldcg(a.bbox_part + i);
-    bb.x = fminf(bb.x, q.x);
-    bb.y = fminf(bb.y, q.y);
-    bb.z = fmaxf(bb.z, q.z);
-    bb.w = fmaxf(bb.w, q.w);
-    et += __ldcg(a.e_part + i);
+  for (int i0 = threadIdx.x; i0 < (int)gridDim.x; i0 += 16 * kGates) {
+    double v[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      v[r] = i0 + r * kGates < (int)gridDim.x ? __ldcg(a.e_part + i0 + r * kGates) : 0.0;
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (i0 + r * kGates < (int)gridDim.x) et += v[r];
   }
   et = block_sum_double(et);
-  bb.x = -block_max_float(-bb.x);
-  bb.y = -block_max_float(-bb.y);
-  bb.z = block_max_float(bb.z);
-  bb.w = block_max_float(bb.w);
   if (threadIdx.x == 0) {
-    if (a.bbox) {
-      a.bbox[0] = f2ord(bb.x);
-      a.bbox[1] = f2ord(bb.y);
-      a.bbox[2] = f2ord(bb.z);
-      a.bbox[3] = f2ord(bb.w);
-    }
-    if (a.energy) *a.energy = et;
+    *a.energy = et;
     *a.done = 0u;
   }
 }
@@ -253,8 +267,7 @@ int attraction_run(fx_ctx *ctx, fx_design *d, float k, float *out,
 static int step_alloc(fx_design *d, cudaStream_t s) {
   StepWork &w = d->step;
   const size_t nb = ((size_t)d->n + kGates - 1) / kGates;
-  if (w.bbox_part.p && w.bbox_part.n >= nb) return FX_OK;
-  FX_TRY(w.bbox_part.alloc(nb));
+  if (w.e_part.p && w.e_part.n >= nb) return FX_OK;
   FX_TRY(w.e_part.alloc(nb));
   FX_TRY(w.done.alloc(4));
   FX_TRY(w.energy.alloc(4));
@@ -487,7 +500,6 @@ extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
     a.xhi = d->chip_w;
     a.yhi = d->chip_h;
     a.bbox = use_bh ? d->bh.bbox.p : nullptr;
-    a.bbox_part = d->step.bbox_part.p;
     a.e_part = d->step.e_part.p;
     a.done = d->step.done.p;
     a.energy = d->step.energy.p;

@@ -234,13 +234,12 @@ struct CongWork {
 
 // ---- fused attraction/integrate step: cross-block reductions ------------------
 struct StepWork {
-  DevBuf<float4> bbox_part;     // per block {min x, min y, max x, max y}
   DevBuf<double> e_part;        // per block density energy
   DevBuf<unsigned int> done;    // last-block counter
   DevBuf<double> energy;        // result
   template <class F>
   void for_each(F &&f) {
-    f(bbox_part); f(e_part); f(done); f(energy);
+    f(e_part); f(done); f(energy);
   }
 };
 
