@@ -1077,6 +1077,130 @@ bh_walk_kernel(int n, const float2 *__restrict__ spos,
                                     err, term_count, st_node[w], st_mask[w]);
 }
 
+// ---- walk of small designs --------------------------------------------------
+// The group walk bit for bit (the same cells in the same order, each point's
+// terms added in the same order), with eight points to a warp and four lanes
+// to a point, one per child of the popped cell: the four children's loads and
+// terms, a chain of four in the group walk, run side by side, and only the
+// additions, from shuffles, keep their order. With few points the walk is
+// bound by that chain, not by issue: 313 warps of 10k points left half of the
+// schedulers idle. A cell's quad children are loaded with its record, so a
+// pass is one trip to memory. 10k points 69 us (group walk 174), 100k 247
+// (293), 130k 306 (332); at 300k, where issue counts, the group walk's 551
+// wins (729), hence the limit.
+constexpr int kSmallWarps = 4;
+constexpr int kSmallWalkMax = 1 << 17;
+
+template <int Stack>
+__global__ void __launch_bounds__(kSmallWarps * 32)
+bh_small_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__restrict__ perm,
+                     const int4 *__restrict__ qchild, const float4 *__restrict__ node, float k,
+                     float th2, float md2, float2 *__restrict__ force,
+                     unsigned int *__restrict__ err) {
+  // opened cells: their quad children, and the points that opened them
+  __shared__ int4 st_kids[kSmallWarps][Stack + 1];
+  __shared__ unsigned st_mask[kSmallWarps][Stack + 1];
+  const unsigned full = 0xffffffffu, ones = 0x11111111u;  // a bit per point
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int slot = lane & 3, own = lane & ~3;
+  const int base = (blockIdx.x * kSmallWarps + w) * 8;
+  if (base >= n) return;  // warp-uniform
+  const int s = base + (lane >> 2);
+  const bool valid = s < n;
+  const float2 p = valid ? spos[s] : make_float2(0.f, 0.f);
+  float fx = 0.f, fy = 0.f;
+  int sp = 0;
+  int4 kids = make_int4(kNone, kNone, kNone, kNone);  // of the lane's child
+  // the opening rule of lane's child c for its point, and the point's terms of
+  // the four children in order; returns which points open which child
+  auto eval = [&](int c, bool in) -> unsigned {
+    float dx = 0.f, dy = 0.f, f = 0.f;
+    bool acc = false, op = false, bucket = false;
+    int b = 0, e = -1;
+    if (in) {
+      float r2c, kq = k;
+      if (c < 0) {  // single point ~c
+        const float2 q = spos[~c];
+        dx = __fsub_rn(p.x, q.x);
+        dy = __fsub_rn(p.y, q.y);
+        r2c = fmaxf(__fmaf_rn(dx, dx, __fmul_rn(dy, dy)), md2);
+        acc = ~c != s;
+      } else {
+        const float4 r0 = node[2 * c], r1 = node[2 * c + 1];
+        kids = qchild[c];  // with the record, not after it: one round trip a cell
+        dx = __fsub_rn(__fsub_rn(p.x, r0.x), r0.z);
+        dy = __fsub_rn(__fsub_rn(p.y, r0.y), r0.w);
+        r2c = fmaxf(__fmaf_rn(dx, dx, __fmul_rn(dy, dy)), md2);
+        kq = __fmul_rn(k, fabsf(r1.x));
+        // size^2 < 0 (a node standing for no quad level) is always opened
+        acc = r1.y >= 0.f && r1.y < __fmul_rn(th2, r2c);
+        op = !acc && r1.x > 0.f;
+        bucket = !acc && !op;
+        b = __float_as_int(r1.z);
+        e = __float_as_int(r1.w);
+      }
+      const float inv = bh_rsqrt(r2c);
+      f = __fmul_rn(__fmul_rn(__fmul_rn(kq, inv), inv), inv);
+    }
+    const unsigned b_acc = __ballot_sync(full, acc), b_bk = __ballot_sync(full, bucket);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const float fh = __shfl_sync(full, f, own + h), xh = __shfl_sync(full, dx, own + h),
+                  yh = __shfl_sync(full, dy, own + h);
+      if ((b_acc >> (own + h)) & 1u) {
+        fx = __fmaf_rn(fh, xh, fx);
+        fy = __fmaf_rn(fh, yh, fy);
+      }
+      if (b_bk & (ones << h)) {  // warp-uniform: some point opens child h, a bucket
+        const int bh = __shfl_sync(full, b, own + h), eh = __shfl_sync(full, e, own + h);
+        if ((b_bk >> (own + h)) & 1u)
+          for (int t = bh; t <= eh; ++t)
+            if (t != s) bh_direct<false>(p.x, p.y, spos[t], k, md2, fx, fy);
+        __syncwarp();
+      }
+    }
+    return __ballot_sync(full, op);
+  };
+  if (n >= 2) {
+    // the root, by the first lane of each point (lane 0's point always exists)
+    const unsigned open = eval(0, valid && slot == 0) & ones;
+    if (open) {
+      if (lane == 0) {
+        st_kids[w][0] = kids;
+        st_mask[w][0] = open;
+      }
+      sp = 1;
+    }
+  }
+  __syncwarp();
+  while (sp > 0) {
+    --sp;
+    const int c = reinterpret_cast<const int *>(&st_kids[w][sp])[slot];
+    const unsigned mask = st_mask[w][sp];
+    __syncwarp();
+    const unsigned ob = eval(c, c != kNone && ((mask >> own) & 1u));
+    const unsigned om = (ob >> slot) & ones;  // the points that open this lane's child
+    // pushed in reverse, so that the first opened child is popped first
+    const unsigned opened = __ballot_sync(full, om != 0u) & 0xfu;
+    const int np = __popc(opened);
+    if (sp + np > Stack) {
+      if (lane == 0) atomicOr(err, 1u);
+      break;
+    }
+    // by the first point that opened the child: its lane has the grandchildren
+    if (om != 0u && own == __ffs(om) - 1) {
+      const int at = sp + __popc(opened >> (slot + 1));
+      st_kids[w][at] = kids;
+      st_mask[w][at] = om;
+    }
+    sp += np;
+    __syncwarp();
+  }
+  if (valid && slot == 0) {
+    force[perm[s]] = make_float2(fx, fy);
+  }
+}
+
 // ---- batched walk (FX_BH_FAST) ----------------------------------------------
 // The same cells, decisions and terms as the group walk, organised by cell
 // instead of by point. Each warp owns 32 consecutive sorted points and a
@@ -1114,7 +1238,10 @@ __device__ __forceinline__ float rsqrt_approx_ftz(float x) {
   return y;
 }
 
-constexpr int kBatchWarps = 8;
+// Blocks of eight warps; of two where eight would leave SMs empty (49 us at 10k
+// points instead of 51).
+constexpr int kBatchWarps = 8, kBatchWarpsFew = 2;
+constexpr int kBatchSpread = 148 * 8 * 32;
 constexpr int kBatchStack = 200;
 
 // The stacked cells a warp may use (kBatchStack; less when the environment
@@ -1176,18 +1303,18 @@ struct BatchSmem {
 static_assert(kBatchStack * sizeof(int4) >= 2 * kWalkGroups * (kStackDeep + 1) * sizeof(int32_t),
               "the group walk's stacks must fit in a warp's batch stack");
 
-template <int Stack, bool Count>
-__global__ void __launch_bounds__(kBatchWarps * 32, 5)
+template <int Stack, bool Count, int Warps>
+__global__ void __launch_bounds__(Warps * 32, 40 / Warps)
 bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__restrict__ perm,
                      const int4 *__restrict__ qchild, const float4 *__restrict__ node,
                      float k, float th2, float md2, float2 *__restrict__ force,
                      unsigned int *__restrict__ err, int32_t *__restrict__ term_count,
                      int stack_cap) {
-  __shared__ __align__(16) BatchSmem smem[kBatchWarps];
+  __shared__ __align__(16) BatchSmem smem[Warps];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   BatchSmem &sh = smem[w];
-  const int base = (blockIdx.x * kBatchWarps + w) * 32;
+  const int base = (blockIdx.x * Warps + w) * 32;
   if (base >= n) return;  // warp-uniform
   const int s = base + lane;
   const bool valid = s < n;
@@ -1586,7 +1713,15 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
   FX_CHECK_LAUNCH();
   timer_end(ctx, FX_STAGE_BH_TREE, s, ev);
   timer_begin(ctx, FX_STAGE_BH_WALK, s, &ev);
-  if (walk == FX_BH_EXACT) {
+  if (walk == FX_BH_EXACT && n <= kSmallWalkMax) {
+    const int wb = (n + kSmallWarps * 8 - 1) / (kSmallWarps * 8);
+    if (deep)
+      bh_small_walk_kernel<kStackDeep><<<wb, kSmallWarps * 32, 0, s>>>(
+          n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err);
+    else
+      bh_small_walk_kernel<kStack><<<wb, kSmallWarps * 32, 0, s>>>(
+          n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err);
+  } else if (walk == FX_BH_EXACT) {
     const int wb = (n + kWalkWarps * 32 - 1) / (kWalkWarps * 32);
     if (deep)
       bh_walk_kernel<kStackDeep><<<wb, kWalkWarps * 32, 0, s>>>(
@@ -1595,9 +1730,11 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
       bh_walk_kernel<kStack><<<wb, kWalkWarps * 32, 0, s>>>(
           n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err);
   } else {
-    const int wb = (n + kBatchWarps * 32 - 1) / (kBatchWarps * 32);
-#define FX_FAST_WALK(ST, CNT)                                                             \
-  bh_batch_walk_kernel<ST, CNT><<<wb, kBatchWarps * 32, 0, s>>>(                          \
+    const int bw = n <= kBatchSpread ? kBatchWarpsFew : kBatchWarps;
+    const int wb = (n + bw * 32 - 1) / (bw * 32);
+#define FX_FAST_WALK(ST, CNT)                                                               \
+  (bw == kBatchWarps ? bh_batch_walk_kernel<ST, CNT, kBatchWarps>                           \
+                     : bh_batch_walk_kernel<ST, CNT, kBatchWarpsFew>)<<<wb, bw * 32, 0, s>>>( \
       n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err, term_count, \
       batch_stack_cap())
     if (deep) {

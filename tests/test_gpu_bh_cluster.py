@@ -19,7 +19,7 @@ def _points(kind, n, rng):
     return c * 50.0 + rng.integers(0, 3, n) * 1e-3, c * 31.0
 
 
-@pytest.mark.parametrize("n", [1, 2, 33, 511, 513, 4096, 4097, 8193, 16384, 16385, 32767, 32768,
+@pytest.mark.parametrize("n", [1, 2, 7, 9, 33, 511, 513, 4096, 4097, 8193, 16384, 16385, 32767, 32768,
                                32769, 65537, 131073])
 @pytest.mark.parametrize("kind", ["uniform", "line", "few"])
 def test_cluster_sort_and_tree(fx, ctx, oracle, n, kind):
