@@ -380,19 +380,75 @@ int radix_sort_tiles(int n) { return (n + kSortTile - 1) / kSortTile; }
 constexpr uint32_t kOsAgg = 1u << 30, kOsInc = 2u << 30, kOsVal = (1u << 30) - 1u;
 constexpr uint32_t kOsSpin = 1u << 22;
 constexpr int kOsWin = 16;  // earlier tiles read per look-back step
-// 4096-key tiles: the look-back chain (one round trip per kOsWin tiles
-// whose predecessors have not finished) is half as long as with 2048.
-constexpr int kOsItems = 16;
-constexpr int kOsTile = kSortThreads * kOsItems;
-static int os_tiles(int n) { return (n + kOsTile - 1) / kOsTile; }
+// Tiles of 512 threads and 4 or 8 keys each: a block's time is mostly its
+// chain of ranking rounds (one per key of a thread) and its look-back, so few
+// keys win while the tiles are few, and long tiles once the look-back is the
+// longer of the two. Keys and sort at 100k points: 51 us with 4, 61 with 8 (84
+// with 256 threads of 16, and root, counts and identity values as launches and
+// arrays of their own); at 1M 126 and 119 (136); even at about 500k.
+constexpr int kOsThreads = 512;
+constexpr int kOsFew = 1 << 19;
+static int os_items(int n) { return n <= kOsFew ? 4 : 8; }
+static int os_tiles(int n) {
+  const int tile = kOsThreads * os_items(n);
+  return (n + tile - 1) / tile;
+}
 
-__global__ void __launch_bounds__(kSortThreads)
+// Root square, keys and every pass's digit counts in one pass over the
+// positions (hist: 4 x 256 counts, zeroed before). Root and counts as launches
+// of their own cost 14 us at 100k points.
+constexpr int kKeysPer = 4;  // points per thread
+
+__global__ void __launch_bounds__(256)
+bh_keys_hist_kernel(const float *__restrict__ x, const float *__restrict__ y, int n,
+                    const unsigned int *__restrict__ bbox, float th2, float md2,
+                    float *__restrict__ root, uint32_t *__restrict__ keys,
+                    uint32_t *__restrict__ hist) {
+  __shared__ uint32_t h[4][256];
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) h[q][t] = 0;
+  const float4 rt = bh_root_of(bbox, th2, md2);
+  if (blockIdx.x == 0 && t == 0) {
+    root[0] = rt.x;
+    root[1] = rt.y;
+    root[2] = rt.z;
+    root[3] = rt.w;
+  }
+  const int b0 = blockIdx.x * (256 * kKeysPer) + t;
+  float px[kKeysPer], py[kKeysPer];
+#pragma unroll
+  for (int r = 0; r < kKeysPer; ++r) {
+    const int i = b0 + r * 256;
+    px[r] = i < n ? x[i] : 0.f;
+    py[r] = i < n ? y[i] : 0.f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kKeysPer; ++r) {
+    const int i = b0 + r * 256;
+    if (i >= n) break;
+    const uint32_t k = (spread15(quantize15(px[r], rt.x, rt.z)) << 1) |
+                       spread15(quantize15(py[r], rt.y, rt.z));
+    keys[i] = k;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) atomicAdd(&h[q][(k >> (8 * q)) & 255u], 1u);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t c = h[q][t];
+    if (c) atomicAdd(hist + q * 256 + t, c);
+  }
+}
+
+__global__ void __launch_bounds__(256)
 os_hist_kernel(const uint32_t *__restrict__ keys, int n, int passes,
                uint32_t *__restrict__ hist) {
   __shared__ uint32_t h[4][256];
-  for (int i = threadIdx.x; i < 4 * 256; i += kSortThreads) (&h[0][0])[i] = 0;
+  for (int i = threadIdx.x; i < 4 * 256; i += 256) (&h[0][0])[i] = 0;
   __syncthreads();
-  for (int i = blockIdx.x * kSortThreads + threadIdx.x; i < n; i += gridDim.x * kSortThreads) {
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
     const uint32_t k = keys[i];
     for (int q = 0; q < passes; ++q) atomicAdd(&h[q][(k >> (8 * q)) & 255u], 1u);
   }
@@ -403,42 +459,29 @@ os_hist_kernel(const uint32_t *__restrict__ keys, int n, int passes,
   }
 }
 
-__global__ void __launch_bounds__(kSortThreads, 3)
+// iin null: the values are the places (the first pass of an unsorted batch).
+template <int kOsItems>
+__global__ void __launch_bounds__(kOsThreads)
 os_pass_kernel(const uint32_t *__restrict__ kin, const int32_t *__restrict__ iin,
                uint32_t *__restrict__ kout, int32_t *__restrict__ iout, int n, int shift,
                const uint32_t *__restrict__ hist, uint32_t *__restrict__ status,
                unsigned int *__restrict__ ticket, unsigned int *__restrict__ err,
                const float *__restrict__ px, const float *__restrict__ py,
                float2 *__restrict__ spos) {
-  constexpr int kWarps = kSortThreads / 32;
-  __shared__ uint32_t cnt[kWarps][256];
-  __shared__ uint32_t tstart[256], gbase[256], ws[kWarps];
+  constexpr int kWarps = kOsThreads / 32, kOsTile = kOsThreads * kOsItems;
+  __shared__ __align__(16) uint16_t cnt[kWarps][256];  // a warp ranks 32 * kOsItems pairs
+  __shared__ uint32_t tstart[256], gbase[256], ws[8], ws2[8];
   __shared__ int tile_s;
   __shared__ uint32_t sk[kOsTile];
   __shared__ int32_t sv[kOsTile];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   if (t == 0) tile_s = (int)atomicAdd(ticket, 1u);
-  for (int i = t; i < kWarps * 256; i += kSortThreads) (&cnt[0][0])[i] = 0;
+  for (int i = t; i < kWarps * 32; i += kOsThreads)
+    reinterpret_cast<uint4 *>(&cnt[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
+  // threads 0 .. 255 own a digit each: its count over all keys
+  const uint32_t dcount = t < 256 ? hist[t] : 0u;
   __syncthreads();
   const int tile = tile_s;
-  // base of every digit: exclusive scan of this pass's digit counts
-  uint32_t dbase;
-  {
-    const uint32_t c = hist[t];
-    uint32_t v = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += u;
-    }
-    if (lane == 31) ws[w] = v;
-    __syncthreads();
-    dbase = v - c;
-    for (int q = 0; q < w; ++q) dbase += ws[q];
-    __syncthreads();
-  }
-  // stable ranks within the tile: per warp by __match_any_sync, then warps
-  // in order (as radix_scatter_kernel)
   const int base = tile * kOsTile + w * (32 * kOsItems);
   const unsigned lt_mask = (1u << lane) - 1u;
   uint32_t k[kOsItems];
@@ -447,91 +490,67 @@ os_pass_kernel(const uint32_t *__restrict__ kin, const int32_t *__restrict__ iin
 #pragma unroll
   for (int r = 0; r < kOsItems; ++r) {
     const int i = base + r * 32 + lane;
-    const bool valid = i < n;
-    k[r] = valid ? kin[i] : 0u;
-    v[r] = valid ? iin[i] : 0;
+    k[r] = i < n ? kin[i] : 0u;
+    v[r] = i < n ? (iin ? iin[i] : i) : 0;
+  }
+  // stable ranks within the tile: per warp by __match_any_sync, then warps
+  // in order (as radix_scatter_kernel)
+#pragma unroll
+  for (int r = 0; r < kOsItems; ++r) {
+    const bool valid = base + r * 32 + lane < n;
     const uint32_t dg = valid ? ((k[r] >> shift) & 255u) : 256u;
     const unsigned peers = __match_any_sync(0xffffffffu, dg);
     const int leader = __ffs(peers) - 1;
     const uint32_t old = valid ? cnt[w][dg] : 0u;
     __syncwarp();
-    if (valid && lane == leader) cnt[w][dg] = old + __popc(peers);
+    if (valid && lane == leader) cnt[w][dg] = (uint16_t)(old + __popc(peers));
     __syncwarp();
     rank[r] = old + __popc(peers & lt_mask);
   }
   __syncthreads();
-  // thread t = digit t: warp offsets within the digit, the digit's count in
-  // this tile, and its start within the tile
-  uint32_t local;
-  {
-    uint32_t run = 0;
+  // digit t: warp offsets, the digit's count in this tile, its start within
+  // the tile and (scan of the counts over all keys) within the output
+  uint32_t local = 0, inc = 0, dinc = 0;
+  if (t < 256) {
+    uint32_t c[kWarps];
+#pragma unroll
+    for (int ww = 0; ww < kWarps; ++ww) c[ww] = cnt[ww][t];
 #pragma unroll
     for (int ww = 0; ww < kWarps; ++ww) {
-      const uint32_t c = cnt[ww][t];
-      cnt[ww][t] = run;
-      run += c;
+      cnt[ww][t] = (uint16_t)local;
+      local += c[ww];
     }
-    local = run;
-    uint32_t x = run;
+    atomicExch(status + (size_t)tile * 256 + t, (tile == 0 ? kOsInc : kOsAgg) | local);
+    inc = local;
+    dinc = dcount;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += u;
-    }
-    if (lane == 31) ws[w] = x;
-    __syncthreads();
-    uint32_t st = x - run;
-    for (int q = 0; q < w; ++q) st += ws[q];
-    tstart[t] = st;
-  }
-  // decoupled look-back for digit t
-  {
-    volatile uint32_t *stv = status;
-    uint32_t *my = status + (size_t)tile * 256 + t;
-    if (tile == 0) {
-      atomicExch(my, kOsInc | local);
-      gbase[t] = dbase - tstart[t];
-    } else {
-      atomicExch(my, kOsAgg | local);
-      // The words of the kOsWin nearest earlier tiles are loaded together
-      // (independent loads, one round trip) and added from the nearest on,
-      // up to the first inclusive one; a tile that has not published yet is
-      // waited for (bounded), then the window restarts from it.
-      uint32_t prefix = 0;
-      uint32_t spin = 0;
-      for (int p = tile - 1; p >= 0;) {
-        uint32_t wv[kOsWin];
-#pragma unroll
-        for (int q = 0; q < kOsWin; ++q)
-          wv[q] = p - q >= 0 ? (uint32_t)stv[(size_t)(p - q) * 256 + t] : (uint32_t)(2u << 30);  // before tile 0: inclusive 0
-        int q = 0;
-        bool done = false;
-#pragma unroll
-        for (int r = 0; r < kOsWin; ++r) {
-          if (done || q < r) continue;  // stopped at an earlier entry
-          const uint32_t flag = wv[r] & ~kOsVal;
-          if (flag == 0u) break;         // not published yet: q == r
-          prefix += wv[r] & kOsVal;
-          q = r + 1;
-          if (flag == kOsInc) done = true;
-        }
-        if (done) break;
-        p -= q;
-        if (q < kOsWin && p >= 0) {  // wait for tile p to publish
-          while ((stv[(size_t)p * 256 + t] & ~kOsVal) == 0u && spin < kOsSpin) ++spin;
-          if (spin >= kOsSpin) {  // expired: record it and stop
-            atomicOr(err, 4u);
-            break;
-          }
-        }
+      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      const uint32_t ud = __shfl_up_sync(0xffffffffu, dinc, o);
+      if (lane >= o) {
+        inc += u;
+        dinc += ud;
       }
-      __threadfence();
-      atomicExch(my, kOsInc | (prefix + local));
-      gbase[t] = dbase + prefix - tstart[t];
+    }
+    if (lane == 31) {
+      ws[w] = inc;
+      ws2[w] = dinc;
     }
   }
   __syncthreads();
-  // stage the tile in sorted order, then write it out coalesced
+  if (t < 256) {
+    uint32_t st = inc - local, dbase = dinc - dcount;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      st += q < w ? ws[q] : 0u;
+      dbase += q < w ? ws2[q] : 0u;
+    }
+    tstart[t] = st;
+    gbase[t] = dbase - st;  // completed by the look-back below
+  }
+  __syncthreads();
+  // stage the tile in sorted order (the other warps while the first eight
+  // look back)
 #pragma unroll
   for (int r = 0; r < kOsItems; ++r) {
     const int i = base + r * 32 + lane;
@@ -542,15 +561,57 @@ os_pass_kernel(const uint32_t *__restrict__ kin, const int32_t *__restrict__ iin
       sv[j] = v[r];
     }
   }
+  if (t < 256 && tile > 0) {  // decoupled look-back for digit t
+    volatile uint32_t *stv = status;
+    // The words of the kOsWin nearest earlier tiles are loaded together
+    // (independent loads, one round trip) and added from the nearest on,
+    // up to the first inclusive one; a tile that has not published yet is
+    // waited for (bounded), then the window restarts from it.
+    uint32_t prefix = 0;
+    uint32_t spin = 0;
+    for (int p = tile - 1; p >= 0;) {
+      uint32_t wv[kOsWin];
+#pragma unroll
+      for (int q = 0; q < kOsWin; ++q)
+        wv[q] = p - q >= 0 ? (uint32_t)stv[(size_t)(p - q) * 256 + t] : (uint32_t)(2u << 30);  // before tile 0: inclusive 0
+      int q = 0;
+      bool done = false;
+#pragma unroll
+      for (int r = 0; r < kOsWin; ++r) {
+        if (done || q < r) continue;  // stopped at an earlier entry
+        const uint32_t flag = wv[r] & ~kOsVal;
+        if (flag == 0u) break;         // not published yet: q == r
+        prefix += wv[r] & kOsVal;
+        q = r + 1;
+        if (flag == kOsInc) done = true;
+      }
+      if (done) break;
+      p -= q;
+      if (q < kOsWin && p >= 0) {  // wait for tile p to publish
+        while ((stv[(size_t)p * 256 + t] & ~kOsVal) == 0u && spin < kOsSpin) ++spin;
+        if (spin >= kOsSpin) {  // expired: record it and stop
+          atomicOr(err, 4u);
+          break;
+        }
+      }
+    }
+    __threadfence();
+    atomicExch(status + (size_t)tile * 256 + t, kOsInc | (prefix + local));
+    gbase[t] += prefix;
+  }
   __syncthreads();
   const int m = min(kOsTile, n - tile * kOsTile);
-  for (int j = t; j < m; j += kSortThreads) {
-    const uint32_t key = sk[j];
-    const uint32_t pos = gbase[(key >> shift) & 255u] + (uint32_t)j;
-    const int32_t g = sv[j];
-    kout[pos] = key;
-    iout[pos] = g;
-    if (spos) spos[pos] = make_float2(px[g], py[g]);
+#pragma unroll
+  for (int r = 0; r < kOsItems; ++r) {
+    const int j = r * kOsThreads + t;
+    if (j < m) {
+      const uint32_t key = sk[j];
+      const uint32_t pos = gbase[(key >> shift) & 255u] + (uint32_t)j;
+      const int32_t g = sv[j];
+      kout[pos] = key;
+      iout[pos] = g;
+      if (spos) spos[pos] = make_float2(px[g], py[g]);
+    }
   }
 }
 
@@ -563,6 +624,26 @@ size_t os_sort_words(int n, int passes) {
   return (size_t)passes * 256 + (size_t)passes * os_tiles(n) * 256 + 4;
 }
 
+// The passes of a sort whose digit counts are in ws; v[0] holds the values,
+// or the places themselves when `places`.
+static int os_passes(uint32_t *k[2], int32_t *v[2], int n, int passes, uint32_t *ws,
+                     unsigned int *err, cudaStream_t s, const float *px, const float *py,
+                     float2 *spos, bool places) {
+  const int T = os_tiles(n);
+  uint32_t *hist = ws, *status = ws + passes * 256,
+           *ticket = status + (size_t)passes * T * 256;
+  for (int pass = 0; pass < passes; ++pass) {
+    const int src = pass & 1, dst = src ^ 1;
+    const bool last = pass == passes - 1;
+    (os_items(n) == 4 ? os_pass_kernel<4> : os_pass_kernel<8>)<<<T, kOsThreads, 0, s>>>(
+        k[src], places && pass == 0 ? nullptr : v[src], k[dst], v[dst], n, 8 * pass,
+        hist + 256 * pass, status + (size_t)pass * T * 256, ticket + pass, err, px, py,
+        last ? spos : nullptr);
+  }
+  FX_CHECK_LAUNCH();
+  return FX_OK;
+}
+
 int radix_sort_onesweep(uint32_t *k[2], int32_t *v[2], int n, int passes, uint32_t *ws,
                         unsigned int *err, cudaStream_t s, const float *px,
                         const float *py, float2 *spos) {
@@ -571,22 +652,9 @@ int radix_sort_onesweep(uint32_t *k[2], int32_t *v[2], int n, int passes, uint32
     set_error("radix_sort_onesweep: %d keys / %d passes out of range", n, passes);
     return FX_EINVAL;
   }
-  const int T = os_tiles(n);
-  uint32_t *hist = ws, *status = ws + passes * 256,
-           *ticket = status + (size_t)passes * T * 256;
   FX_CHECK_CUDA(cudaMemsetAsync(ws, 0, os_sort_words(n, passes) * 4, s));
-  const int hb = std::min(T, 2 * 148);
-  os_hist_kernel<<<hb, kSortThreads, 0, s>>>(k[0], n, passes, hist);
-  for (int pass = 0; pass < passes; ++pass) {
-    const int src = pass & 1, dst = src ^ 1;
-    const bool last = pass == passes - 1;
-    os_pass_kernel<<<T, kSortThreads, 0, s>>>(k[src], v[src], k[dst], v[dst], n, 8 * pass,
-                                              hist + 256 * pass,
-                                              status + (size_t)pass * T * 256, ticket + pass,
-                                              err, px, py, last ? spos : nullptr);
-  }
-  FX_CHECK_LAUNCH();
-  return FX_OK;
+  os_hist_kernel<<<std::min((n + 2047) / 2048, 2 * 148), 256, 0, s>>>(k[0], n, passes, ws);
+  return os_passes(k, v, n, passes, ws, err, s, px, py, spos, false);
 }
 
 // ---- exact prefix sums of the sorted positions ---------------------------------
@@ -599,6 +667,7 @@ int radix_sort_onesweep(uint32_t *k[2], int32_t *v[2], int n, int passes, uint32
 // with hi/lo the upper (signed) and lower (unsigned) 64 bits, each step
 // rounded to nearest.
 constexpr int kFixThreads = 256, kFixItems = 8, kFixTile = kFixThreads * kFixItems;
+constexpr int kFixSmall = 1 << 18;  // points up to which tiles hold 512
 
 // Inclusive scan of one int128 per thread over the block; also returns the
 // block total.
@@ -623,13 +692,14 @@ __device__ __forceinline__ __int128 block_scan128(__int128 v, __int128 &total) {
   return v + off;
 }
 
-// The (x, y) sums of each tile of kFixTile sorted points.
+// The (x, y) sums of each tile of 256 * kItems sorted points.
+template <int kItems>
 __global__ void __launch_bounds__(kFixThreads)
 fix_tile_kernel(const float2 *__restrict__ spos, int n, ulonglong4 *__restrict__ tile_sum) {
-  const int b0 = blockIdx.x * kFixTile + threadIdx.x;
+  const int b0 = blockIdx.x * (kFixThreads * kItems) + threadIdx.x;
   FixSums s{0, 0};
 #pragma unroll
-  for (int k = 0; k < kFixItems; ++k) {
+  for (int k = 0; k < kItems; ++k) {
     const int i = b0 + k * kFixThreads;
     if (i < n) {
       const float2 p = spos[i];
@@ -784,10 +854,16 @@ constexpr int kNone = INT_MIN;
 // every node lists up to four, in key order (leaf s as ~s, kNone: empty).
 __global__ void __launch_bounds__(kBuildThreads)
 bh_build_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ slo,
-                const float *__restrict__ root, int n,
+                const float *__restrict__ root, unsigned int *__restrict__ bbox, int n,
                 const ulonglong4 *__restrict__ prefix, float4 *__restrict__ node,
                 int4 *__restrict__ qchild) {
   const int i = blockIdx.x * kBuildThreads + threadIdx.x;
+  if (i == 0) {  // re-armed for the next accumulation (the keys are made)
+    bbox[0] = 0xffffffffu;
+    bbox[1] = 0xffffffffu;
+    bbox[2] = 0u;
+    bbox[3] = 0u;
+  }
   const bool valid = i < n - 1;
   const bool deep = slo && root[3] > 0.f;
   const int kb = deep ? kDeepBits : kKeyBits;  // prefix length of a bucket
@@ -1546,7 +1622,8 @@ static int bh_alloc(fx_design *d) {
   FX_TRY(b.digit_total.alloc(256));
   FX_TRY(b.spos.alloc(n));
   FX_TRY(b.qchild.alloc(ni));
-  FX_TRY(b.tile_fix.alloc(std::max(((size_t)n + kFixTile - 1) / kFixTile, (size_t)64)));
+  FX_TRY(b.tile_fix.alloc(std::max(((size_t)n + kFixTile - 1) / kFixTile,
+                                   ((size_t)std::min(n, kFixSmall) + 511) / 512)));
   FX_TRY(b.prefix.alloc(n));
   FX_TRY(b.node.alloc(2 * ni));
   FX_TRY(b.root.alloc(4));
@@ -1618,18 +1695,36 @@ static int bh_sort_large(fx_ctx *ctx, fx_design *d, const float *x, const float 
   const int T = (n + kSortTile - 1) / kSortTile;
   int launches = 0;
   cudaEvent_t ev;
+  uint32_t *kk[2] = {b.keys[0].p, b.keys[1].p};
+  int32_t *vv[2] = {b.idx[0].p, b.idx[1].p};
   timer_begin(ctx, FX_STAGE_BH_KEYS, s, &ev);
+  if (!deep) {
+    if (n >= (int)kOsVal) {
+      set_error("Barnes-Hut sort: %d points out of range", n);
+      return FX_EINVAL;
+    }
+    FX_CHECK_CUDA(cudaMemsetAsync(b.os_ws.p, 0, os_sort_words(n, 4) * 4, s));
+    bh_keys_hist_kernel<<<(n + 256 * kKeysPer - 1) / (256 * kKeysPer), 256, 0, s>>>(
+        x, y, n, b.bbox.p, th2, md2, b.root.p, b.keys[0].p, b.os_ws.p);
+    FX_CHECK_LAUNCH();
+    timer_end(ctx, FX_STAGE_BH_KEYS, s, ev);
+    timer_begin(ctx, FX_STAGE_BH_SORT, s, &ev);
+    // result in buffer 0; the last pass also gathers the sorted positions
+    FX_TRY(os_passes(kk, vv, n, 4, b.os_ws.p, b.bbox.p + 4, s, x, y, b.spos.p, true));
+    timer_end(ctx, FX_STAGE_BH_SORT, s, ev);
+    ctx->launches += 5;
+    return FX_OK;
+  }
   bh_root_kernel<<<1, 1, 0, s>>>(b.bbox.p, b.root.p, th2, md2);
   FX_CHECK_LAUNCH();
-  bh_keys_kernel<<<gb, 256, 0, s>>>(x, y, n, b.root.p, b.keys[0].p, b.idx[0].p,
-                                    deep ? b.klo.p : nullptr, deep ? b.kl[0].p : nullptr,
-                                    deep ? b.il[0].p : nullptr);
+  bh_keys_kernel<<<gb, 256, 0, s>>>(x, y, n, b.root.p, b.keys[0].p, b.idx[0].p, b.klo.p,
+                                    b.kl[0].p, b.il[0].p);
   FX_CHECK_LAUNCH();
   launches += 2;
   timer_end(ctx, FX_STAGE_BH_KEYS, s, ev);
   timer_begin(ctx, FX_STAGE_BH_SORT, s, &ev);
   const float *gate = b.root.p;
-  if (deep) {
+  {
     // stable sort by the 24-bit sub-key (3 passes; no-ops unless root[3]),
     // then the primary keys and indices in that order into buffer 0
     for (int pass = 0; pass < 3; ++pass) {
@@ -1649,17 +1744,11 @@ static int bh_sort_large(fx_ctx *ctx, fx_design *d, const float *x, const float 
     FX_CHECK_LAUNCH();
     launches += 9 + 2;
   }
-  {
-    uint32_t *kk[2] = {b.keys[0].p, b.keys[1].p};
-    int32_t *vv[2] = {b.idx[0].p, b.idx[1].p};
-    // result in buffer 0; the last pass also gathers the sorted positions
-    FX_TRY(radix_sort_onesweep(kk, vv, n, 4, b.os_ws.p, b.bbox.p + 4, s, x, y, b.spos.p));
-  }
+  // result in buffer 0; the last pass also gathers the sorted positions
+  FX_TRY(radix_sort_onesweep(kk, vv, n, 4, b.os_ws.p, b.bbox.p + 4, s, x, y, b.spos.p));
   launches += 5;
-  if (deep) {
-    bh_deep_slo_kernel<<<gb, 256, 0, s>>>(gate, n, b.klo.p, b.idx[0].p, b.slo.p);
-    ++launches;
-  }
+  bh_deep_slo_kernel<<<gb, 256, 0, s>>>(gate, n, b.klo.p, b.idx[0].p, b.slo.p);
+  ++launches;
   FX_CHECK_LAUNCH();
   timer_end(ctx, FX_STAGE_BH_SORT, s, ev);
   ctx->launches += launches;
@@ -1694,20 +1783,22 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
   }
   timer_begin(ctx, FX_STAGE_BH_TREE, s, &ev);
   if (n >= 2) {
-    // exact prefix sums, from tile sums (the cluster sort makes its own)
-    if (one) {
-      fix_prefix_kernel<2><<<(n + 511) / 512, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p,
-                                                                   b.prefix.p);
+    // exact prefix sums, from tile sums (the cluster sort makes its own);
+    // small tiles spread a small design over the SMs, but a block adds up all
+    // earlier tiles' sums
+    if (n <= kFixSmall) {
+      const int tiles = (n + 511) / 512;
+      if (!one) fix_tile_kernel<2><<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p);
+      fix_prefix_kernel<2><<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p, b.prefix.p);
     } else {
       const int tiles = (n + kFixTile - 1) / kFixTile;
-      fix_tile_kernel<<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p);
+      fix_tile_kernel<kFixItems><<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p);
       fix_prefix_kernel<kFixItems><<<tiles, kFixThreads, 0, s>>>(b.spos.p, n, b.tile_fix.p,
                                                                  b.prefix.p);
-      ++launches;
     }
-    ++launches;
+    launches += one ? 1 : 2;
     bh_build_kernel<<<(n - 1 + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s>>>(
-        b.keys[0].p, deep ? b.slo.p : nullptr, b.root.p, n, b.prefix.p, b.node.p, b.qchild.p);
+        b.keys[0].p, deep ? b.slo.p : nullptr, b.root.p, b.bbox.p, n, b.prefix.p, b.node.p, b.qchild.p);
     ++launches;
   }
   FX_CHECK_LAUNCH();

@@ -43,6 +43,34 @@ def test_cluster_sort_and_tree(fx, ctx, oracle, n, kind):
     assert np.hypot(gx - o["fx"], gy - o["fy"]).sum() <= 1e-5 * ref
 
 
+@pytest.mark.parametrize("n", [262144, 262145, 524288, 524289, 528385])
+def test_many_block_sort(fx, ctx, n):
+    """Past the cluster's capacity: the sizes where tiles of keys and of prefix sums change.
+    Keys and order against a stable sort in numpy; the deep-key path is not taken (die 501)."""
+    rng = np.random.default_rng(n)
+    x, y = (v.astype(np.float32) for v in _points("uniform", n, rng))
+    x[: n // 3] = x[0]  # crowded digits
+    c = fx.Circuit.from_nets([[0, 1]], n, 501.0, 501.0)
+    d = fx.Design(ctx, c)
+    try:
+        d.set_positions(x, y)
+        keys, perm, root = d.barnes_hut(0.5, 0.5, 0.1, walk=fx.FX_BH_FAST)[2:]
+    finally:
+        d.close()
+
+    def cell(v, o):
+        t = (v - o) / root[2] * np.float32(32768)
+        return np.clip(np.ceil(t).astype(np.int64) - 1, 0, 32767).astype(np.uint32)
+
+    def spread(v):
+        for m, k in ((0x00ff00ff, 8), (0x0f0f0f0f, 4), (0x33333333, 2), (0x55555555, 1)):
+            v = (v | (v << np.uint32(k))) & np.uint32(m)
+        return v
+
+    assert np.array_equal(keys, (spread(cell(x, root[0])) << np.uint32(1)) | spread(cell(y, root[1])))
+    assert np.array_equal(perm, np.argsort(keys, kind="stable"))
+
+
 def test_same_point(fx, ctx):
     n = 3000
     c = fx.Circuit.from_nets([[0, 1]], n, 501.0, 501.0)
