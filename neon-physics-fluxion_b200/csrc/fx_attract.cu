@@ -24,6 +24,7 @@ namespace fx {
 
 int bh_bbox(fx_ctx *ctx, fx_design *d, const float *x, const float *y,
             cudaStream_t s);
+int density_prepare(fx_design *d, int G, int precision, cudaStream_t s);
 int density_scatter(fx_ctx *ctx, fx_design *d, const float *x, const float *y,
                     int G, int precision, cudaStream_t s);
 
@@ -430,10 +431,16 @@ extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
   // Bounding box / density of the starting positions; each step then
   // prepares both for the positions it writes.
   auto prologue = [&]() -> int {
-    if (use_bh) FX_TRY(bh_bbox(ctx, d, d->x[d->cur].p, d->y[d->cur].p, s));
-    if (use_dens)
+    // the scatter feeds the density solve alone, so it runs on the second
+    // stream beside the box and the tree (the first step joins it)
+    if (use_dens) {
+      FX_TRY(density_prepare(d, G, c.dct_precision, s));
+      FX_CHECK_CUDA(cudaEventRecord(ctx->fork, s));
+      FX_CHECK_CUDA(cudaStreamWaitEvent(s2, ctx->fork, 0));
       FX_TRY(density_scatter(ctx, d, d->x[d->cur].p, d->y[d->cur].p, G,
-                             c.dct_precision, s));
+                             c.dct_precision, s2));
+    }
+    if (use_bh) FX_TRY(bh_bbox(ctx, d, d->x[d->cur].p, d->y[d->cur].p, s));
     if (use_cong) FX_TRY(congestion_alloc(d, c.cong_cols, c.cong_rows, s));
     return FX_OK;
   };
@@ -613,7 +620,7 @@ extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
       replayed = true;
     }
     it = iters;
-  } else {
+  } else if (iters > 0) {
     FX_TRY(prologue());
   }
   // Long runs replay a CUDA graph of two iterations (one per ping-pong

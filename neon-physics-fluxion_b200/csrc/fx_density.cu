@@ -361,6 +361,13 @@ static int dens_setup(fx_design *d, int G, int precision, cudaStream_t s) {
   return FX_OK;
 }
 
+// Sizes the workspace and builds the tables of a G-bin solve (a no-op when they
+// are there). Call it on the context's primary stream before density_scatter
+// on another.
+int density_prepare(fx_design *d, int G, int precision, cudaStream_t s) {
+  return dens_setup(d, G, precision, s);
+}
+
 // Scatter of the given positions into the area accumulator.
 int density_scatter(fx_ctx *ctx, fx_design *d, const float *x, const float *y,
                     int G, int precision, cudaStream_t s) {

@@ -109,48 +109,45 @@ __device__ __forceinline__ void red_add_global(unsigned long long *p, unsigned l
 // combined and one lane issues the atomic. Every lane of the warp must call
 // these (idx < 0 = nothing to add); base is global memory. Sums of integers
 // are exact, so the result does not depend on the grouping.
-// Groups are taken one by one, the lowest waiting lane's first, while they
-// are of four lanes or more; what is left adds lane by lane. Spread indexes
-// (an early placement) so cost one shuffle and ballot, crowded ones (a
-// contracted placement, whose gates share a few elements) a round per element.
-// __match_any_sync takes a step per distinct value: with it the net kernel,
-// four adds a net, took 67 us instead of 61 at 1M gates (ncu cold), and 500
-// iterations into a contracted placement ran at 1880 a second instead of 2830
-// (with the walk's gain).
-constexpr int kAggFew = 4;
+// Lanes are grouped by __match_any_sync, which takes a step per distinct value,
+// only where two neighbouring lanes name the same element; otherwise they are
+// spread (an early placement: 61 us for the net kernel at 1M gates, whose four
+// adds a net took 67 when always matched, ncu cold) and add lane by lane.
+// Crowded elements (a contracted placement, a grid's corner) nearly always
+// show such a pair, and what is missed costs time only.
+__device__ __forceinline__ bool crowded(int i) {
+  const int next = __shfl_down_sync(0xffffffffu, i, 1);  // by every lane, before any test
+  return __any_sync(0xffffffffu, i >= 0 && i == next && (threadIdx.x & 31u) < 31u);
+}
 
 __device__ __forceinline__ void agg_add_u64(unsigned long long *base, long long idx,
                                             unsigned long long v) {
-  // indexes fit 31 bits (density bins: G^2 <= 8192^2)
-  const int i = (int)idx;
   const unsigned lane = threadIdx.x & 31u;
-  unsigned todo = __ballot_sync(0xffffffffu, i >= 0);
-  while (todo) {
-    const int lead = __ffs(todo) - 1;
-    const unsigned m = __ballot_sync(0xffffffffu, i == __shfl_sync(0xffffffffu, i, lead));
-    if (__popc(m) < kAggFew) break;
-    unsigned long long sum = (m >> lane) & 1u ? v : 0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((int)lane == lead) red_add_global(base + i, sum);
-    todo &= ~m;
+  const int i = (int)idx;  // indexes fit 31 bits (density bins: G^2 <= 8192^2)
+  if (!crowded(i)) {
+    if (i >= 0) red_add_global(base + i, v);
+    return;
   }
-  if ((todo >> lane) & 1u) red_add_global(base + i, v);
+  const unsigned peers = __match_any_sync(0xffffffffu, i);
+  unsigned long long sum = 0;
+#pragma unroll
+  for (int src = 0; src < 32; ++src) {
+    const unsigned long long w = __shfl_sync(0xffffffffu, v, src);
+    if ((peers >> src) & 1u) sum += w;
+  }
+  if (i >= 0 && lane == (unsigned)(__ffs(peers) - 1)) red_add_global(base + i, sum);
 }
 
 // Adds the same constant `v` from every lane naming idx (>= 0).
 __device__ __forceinline__ void agg_add_const_i32(int *base, long long idx, int v) {
-  const int i = (int)idx;  // indexes fit 31 bits
   const unsigned lane = threadIdx.x & 31u;
-  unsigned todo = __ballot_sync(0xffffffffu, i >= 0);
-  while (todo) {
-    const int lead = __ffs(todo) - 1;
-    const unsigned m = __ballot_sync(0xffffffffu, i == __shfl_sync(0xffffffffu, i, lead));
-    if (__popc(m) < kAggFew) break;
-    if ((int)lane == lead) red_add_global(base + i, v * __popc(m));
-    todo &= ~m;
+  const int i = (int)idx;  // indexes fit 31 bits
+  if (!crowded(i)) {
+    if (i >= 0) red_add_global(base + i, v);
+    return;
   }
-  if ((todo >> lane) & 1u) red_add_global(base + i, v);
+  const unsigned peers = __match_any_sync(0xffffffffu, i);
+  if (i >= 0 && lane == (unsigned)(__ffs(peers) - 1)) red_add_global(base + i, v * __popc(peers));
 }
 
 // Order-preserving float <-> uint mapping for atomicMin/atomicMax.
