@@ -1298,10 +1298,10 @@ bh_small_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__re
 // Opened cells push their quad children with the opening lanes as the mask;
 // opened buckets are walked point by point. Per point the interaction list is
 // exactly the group walk's; the terms are added in another order.
-// Issue-bound (78 % issue-active, ALU pipe 63 %): of the 613 entries of a warp
+// Issue-bound (75 % issue-active, ALU pipe 58 %): of the 613 entries of a warp
 // at 1M uniform points 125 are accepted by all, 272 by a mask, 159 tested and
 // 57 opened by all; testing every entry for every lane took 0.66 ms and
-// 604M warp instructions, this 0.57 ms and 476M (300k points: 0.217, 0.198 ms).
+// 604M warp instructions, this 0.52 ms and 426M (300k points: 0.217, 0.174 ms).
 // The stack holds kBatchStack cells (of up to four children; in a CPU model
 // of this walk the children of uniform, clustered, line and radial sets of
 // 20k-1M points peaked at 160-224): a warp whose stack would overflow starts over with
@@ -1314,10 +1314,6 @@ __device__ __forceinline__ float rsqrt_approx_ftz(float x) {
   return y;
 }
 
-// Blocks of eight warps; of two where eight would leave SMs empty (49 us at 10k
-// points instead of 51).
-constexpr int kBatchWarps = 8, kBatchWarpsFew = 2;
-constexpr int kBatchSpread = 148 * 8 * 32;
 constexpr int kBatchStack = 200;
 
 // The stacked cells a warp may use (kBatchStack; less when the environment
@@ -1379,19 +1375,22 @@ struct BatchSmem {
 static_assert(kBatchStack * sizeof(int4) >= 2 * kWalkGroups * (kStackDeep + 1) * sizeof(int32_t),
               "the group walk's stacks must fit in a warp's batch stack");
 
-template <int Stack, bool Count, int Warps>
-__global__ void __launch_bounds__(Warps * 32, 40 / Warps)
+// Blocks of one warp: its shared memory then lies at fixed addresses, which
+// saves the instructions that find a warp's part of a block's (0.52 ms at 1M
+// points against 0.56 and 0.57 with blocks of two and eight), and small
+// designs reach every SM (43 against 47 us at 5k). 64 registers allow the SM
+// all of the 32 blocks it can hold.
+template <int Stack, bool Count>
+__global__ void __launch_bounds__(32)
 bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__restrict__ perm,
                      const int4 *__restrict__ qchild, const float4 *__restrict__ node,
                      float k, float th2, float md2, float2 *__restrict__ force,
                      unsigned int *__restrict__ err, int32_t *__restrict__ term_count,
                      int stack_cap) {
-  __shared__ __align__(16) BatchSmem smem[Warps];
+  __shared__ __align__(16) BatchSmem sh;
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  BatchSmem &sh = smem[w];
-  const int base = (blockIdx.x * Warps + w) * 32;
-  if (base >= n) return;  // warp-uniform
+  const int lane = threadIdx.x;
+  const int base = blockIdx.x * 32;
   const int s = base + lane;
   const bool valid = s < n;
   const unsigned lanebit = 1u << lane, lt = lanebit - 1u;
@@ -1821,11 +1820,9 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
       bh_walk_kernel<kStack><<<wb, kWalkWarps * 32, 0, s>>>(
           n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err);
   } else {
-    const int bw = n <= kBatchSpread ? kBatchWarpsFew : kBatchWarps;
-    const int wb = (n + bw * 32 - 1) / (bw * 32);
-#define FX_FAST_WALK(ST, CNT)                                                               \
-  (bw == kBatchWarps ? bh_batch_walk_kernel<ST, CNT, kBatchWarps>                           \
-                     : bh_batch_walk_kernel<ST, CNT, kBatchWarpsFew>)<<<wb, bw * 32, 0, s>>>( \
+    const int wb = (n + 31) / 32;
+#define FX_FAST_WALK(ST, CNT)                                                             \
+  bh_batch_walk_kernel<ST, CNT><<<wb, 32, 0, s>>>(                                        \
       n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err, term_count, \
       batch_stack_cap())
     if (deep) {

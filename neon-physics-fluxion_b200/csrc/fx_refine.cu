@@ -74,6 +74,18 @@ __device__ __forceinline__ int2 total_clip(int2 a) {
   return make_int2(min(a.x, kTotalSat), min(a.y, kTotalSat));
 }
 
+// Inclusive composition over the first kN lanes of the warp.
+template <int kN>
+__device__ __forceinline__ int2 total_scan(int2 v, int lane) {
+#pragma unroll
+  for (int o = 1; o < kN; o <<= 1) {
+    const int2 before = make_int2(__shfl_up_sync(0xffffffffu, v.x, o),
+                                  __shfl_up_sync(0xffffffffu, v.y, o));
+    if (lane >= o) v = total_then(before, v);
+  }
+  return v;
+}
+
 __global__ void __launch_bounds__(kTotalThreads)
 refine_total_kernel(const uint32_t *__restrict__ counts, int cells, float cap, float threshold,
                     int decide, RefineState *__restrict__ st, RefineState *__restrict__ host) {
@@ -157,47 +169,44 @@ refine_total_kernel(const uint32_t *__restrict__ counts, int cells, float cap, f
         sum += t[r].x;
         tie |= t[r].x != t[r].y;
       }
-      // inclusive scan of the maps over the warp: plain sums unless one of
-      // its terms ties
-      int2 inc;
-      if (!__any_sync(0xffffffffu, tie)) {
-        int v = min(sum, kTotalSat);
+      // the chunk's map: the warps' totals (plain sums unless a term ties),
+      // composed in order. No scan yet: most chunks stay in their binade.
+      const bool warp_tie = __any_sync(0xffffffffu, tie);
+      int2 d = make_int2(sum, sum);
+      if (warp_tie) {
+        d = t[0];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, v, o);
-          if (lane >= o) v += u;
-        }
-        inc = make_int2(v, v);
+        for (int r = 1; r < kTotalItems; ++r) d = total_then(d, t[r]);
+      }
+      d = total_clip(d);
+      int2 inc = d;  // of the warp, valid in its last lane
+      if (!warp_tie) {
+        const int all = __reduce_add_sync(0xffffffffu, d.x);
+        inc = make_int2(all, all);
       } else {
-        inc = t[0];
-#pragma unroll
-        for (int r = 1; r < kTotalItems; ++r) inc = total_then(inc, t[r]);
-        inc = total_clip(inc);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int2 before = make_int2(__shfl_up_sync(0xffffffffu, inc.x, o),
-                                        __shfl_up_sync(0xffffffffu, inc.y, o));
-          if (lane >= o) inc = total_then(before, inc);
-        }
+        inc = total_scan<32>(d, lane);
       }
       inc = total_clip(inc);
       if (lane == 31) wsum[w] = inc;
       if (tid == 0) cross_sh = INT_MAX;
       __syncthreads();
       int2 wi = lane < kTotalWarps ? wsum[lane] : make_int2(0, 0);
-#pragma unroll
-      for (int o = 1; o < kTotalWarps; o <<= 1) {
-        const int2 before = make_int2(__shfl_up_sync(0xffffffffu, wi.x, o),
-                                      __shfl_up_sync(0xffffffffu, wi.y, o));
-        if (lane >= o) wi = total_then(before, wi);
-      }
       const int odd = S0 & 1;
-      const int all = __shfl_sync(0xffffffffu, odd ? wi.y : wi.x, kTotalWarps - 1);
+      int all;
+      const bool block_tie = __any_sync(0xffffffffu, wi.x != wi.y);
+      if (!block_tie) {
+        all = __reduce_add_sync(0xffffffffu, wi.x);
+      } else {
+        const int2 c = total_scan<kTotalWarps>(wi, lane);
+        all = __shfl_sync(0xffffffffu, odd ? c.y : c.x, kTotalWarps - 1);
+      }
       if (S0 + all < kTotalFull) {  // the chunk ends in this binade
         if (!small) s = __fmul_rn((float)(S0 + all), __int_as_float((127 + e - 23) << 23));
         __syncthreads();  // wsum and cross_sh are free again
         break;
       }
+      inc = total_scan<32>(d, lane);
+      wi = total_scan<kTotalWarps>(wi, lane);
       // the first term that takes S to 2^24, by the thread that holds it
       const int2 wex = make_int2(__shfl_sync(0xffffffffu, wi.x, max(w - 1, 0)),
                                  __shfl_sync(0xffffffffu, wi.y, max(w - 1, 0)));
