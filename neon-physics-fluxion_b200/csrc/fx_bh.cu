@@ -1306,14 +1306,6 @@ bh_small_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__re
 // of this walk the children of uniform, clustered, line and radial sets of
 // 20k-1M points peaked at 160-224): a warp whose stack would overflow starts over with
 // the group walk, whose stacks are bounded, in the same shared memory.
-// The hardware reciprocal square root without the subnormal handling of
-// rsqrtf (the argument here is at least min_dist^2).
-__device__ __forceinline__ float rsqrt_approx_ftz(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 constexpr int kBatchStack = 200;
 
 // The stacked cells a warp may use (kBatchStack; less when the environment
@@ -1326,33 +1318,6 @@ static int batch_stack_cap() {
     return std::min(kBatchStack, std::max(4, v));
   }();
   return cap;
-}
-
-// Packed pairs of f32 (one instruction, each half rounded as the scalar one).
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
 }
 
 // Two entries side by side, one half of each packed register: -x and -y of

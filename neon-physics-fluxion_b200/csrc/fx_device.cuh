@@ -150,6 +150,41 @@ __device__ __forceinline__ void agg_add_const_i32(int *base, long long idx, int 
   if (i >= 0 && lane == (unsigned)(__ffs(peers) - 1)) red_add_global(base + i, v * __popc(peers));
 }
 
+// The hardware reciprocal square root without the subnormal handling of
+// rsqrtf, for arguments that are never subnormal.
+__device__ __forceinline__ float rsqrt_approx_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Packed pairs of f32 (one instruction, each half rounded as the scalar one).
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 // Order-preserving float <-> uint mapping for atomicMin/atomicMax.
 __device__ __forceinline__ unsigned int f2ord(float f) {
   const unsigned int u = __float_as_uint(f);
