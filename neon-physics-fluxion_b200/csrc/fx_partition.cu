@@ -27,6 +27,7 @@
 //                  quotient), per-cluster stop once the Rayleigh quotient
 //                  changes by <= tol (relative), at most power_iterations.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <vector>
 
@@ -381,98 +382,239 @@ __global__ void part_combine_kernel(int C, const int32_t *__restrict__ beg,
 }
 
 // ---- fixed iteration counts on clusters of several chunks --------------------
-// Two launches an iteration instead of four: the chunk sums with the
-// per-cluster combination in the last block to finish, and a product that
-// normalises its inputs as it reads them (v_j = (x_j - mean) / norm, a
-// division per neighbour, but no pass of its own over the vector). 22 us an
-// iteration at 100k gates against 37 (ncu cold); bound by the latency of the
-// sums' chain and of the gathers.
-constexpr int kSumThreads = 512;
+// Every power iteration of a depth in one cooperative launch. Per iteration:
+// a block per chunk sums it (part), all blocks meet, each combines the chunks
+// of the clusters its own positions lie in, multiplies (the inputs normalised
+// as they are read, v_j = (x_j - mean) / norm: a division per neighbour, but
+// no pass of its own over the vector), and all meet again. At 100k gates an
+// iteration takes 7 to 10 us (22 with two launches each, whose longest rows,
+// 129 neighbours in sequence, set the time): sums 2, meetings 1.5 each, the
+// combination 1.3, the product 1.5 to 4. Bound by L2 round trips and a lane's
+// 128 dependent FP64 sums. Blocks get even shares of positions and neighbours,
+// not of positions: the order by Fiedler value gathers the hubs at the ends
+// (9.9 us a product by positions, 4.3 by shares). A hierarchy of 100k gates
+// takes 3.7 ms (5.4 before), of 1M 17.2.
+constexpr int kPowerThreads = 512;
+constexpr int kPowerClusters = 1024;      // clusters the positions of a block may span
+constexpr int kPowerTile = kPartChunk / 4;  // chunk sums staged at a time
+constexpr int kPowerEdges = 8192;           // neighbours gathered at a time
+static_assert(kPowerEdges >= 2 * kPartChunk, "buf holds a chunk in FP64");
+constexpr int kPowerPos = 8;  // work of a position, in neighbours
+constexpr int kPowerSmem = 2 * kPowerEdges * 4;
+constexpr int kMeetSpin = 1 << 22;        // polls before a block gives up (seconds)
 
-__global__ void __launch_bounds__(kSumThreads)
-part_sums_kernel(int C, const int32_t *__restrict__ ck_beg, const int32_t *__restrict__ ck_end,
-                 const int32_t *__restrict__ cl_ck, const int32_t *__restrict__ beg,
-                 const int32_t *__restrict__ end, const float *__restrict__ x, int deflate,
-                 double *__restrict__ part, unsigned int *__restrict__ done,
-                 float *__restrict__ mean, float *__restrict__ nrm) {
-  // the block brings its chunk to shared memory in one round of loads; then
-  // warp 0 sums x and warp 1 x^2 (a lane's 128 sums are a chain)
-  __shared__ float buf[kPartChunk];
-  const int k = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int b = ck_beg[k], n = ck_end[k] - b;
-  float v[kPartChunk / kSumThreads];
-#pragma unroll
-  for (int r = 0; r < kPartChunk / kSumThreads; ++r) {
-    const int i = r * kSumThreads + threadIdx.x;
-    v[r] = i < n ? x[b + i] : 0.f;
-  }
-#pragma unroll
-  for (int r = 0; r < kPartChunk / kSumThreads; ++r) buf[r * kSumThreads + threadIdx.x] = v[r];
+// Every block arrives and waits for the others, which a cooperative launch
+// keeps resident; sync[0] counts arrivals (target: those so far and this
+// meeting's), sync[1] is set by a block that gave up. True if all went well.
+__device__ bool all_meet(unsigned int *sync, unsigned int target) {
   __syncthreads();
-  if (w < 2) {
-    double s = 0.0;
-    if (w == 0) {
-#pragma unroll 8
-      for (int i = lane; i < n; i += 32) s += (double)buf[i];
-    } else {
-#pragma unroll 8
-      for (int i = lane; i < n; i += 32) {
-        const double a = (double)buf[i];
-        s += a * a;
-      }
-    }
-    s = tree_sum(s);
-    if (lane == 0) part[3 * k + w] = s;
+  bool bad = false;
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sync) : "memory");
+    int spin = 0;
+    unsigned int seen;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync) : "memory");
+    } while ((int)(seen - target) < 0 && ++spin < kMeetSpin);
+    bad = spin >= kMeetSpin;
+    if (bad) atomicExch(sync + 1, 1u);
   }
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    double s1 = 0.0, s2 = 0.0;
-    for (int q = cl_ck[c]; q < cl_ck[c + 1]; ++q) {
-      s1 += __ldcg(part + 3 * q);
-      s2 += __ldcg(part + 3 * q + 1);
-    }
-    mean_norm(s1, s2, (double)(end[c] - beg[c]), deflate, mean[c], nrm[c]);
-  }
-  if (threadIdx.x == 0) *done = 0u;
+  return !__syncthreads_or(bad);
 }
 
-// v = normed(x) and lv = L v, in the order of part_spmv_csr_kernel.
-__global__ void part_step_kernel(int n, const int32_t *__restrict__ rp,
-                                 const int32_t *__restrict__ col,
-                                 const int32_t *__restrict__ clp,
-                                 const float *__restrict__ deg, const float *__restrict__ mean,
-                                 const float *__restrict__ nrm, const float *__restrict__ x,
-                                 float *__restrict__ v, float *__restrict__ lv) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int c = clp[p];
-  if (c < 0) return;
-  const float m = mean[c], r = nrm[c];
-  const float vp = normed(x[p], m, r);
-  v[p] = vp;
-  float l = __fmul_rn(deg[p], vp);
-  const int e1 = rp[p + 1];
-  // eight neighbours' loads and divisions in flight, subtracted in order
-  for (int e = rp[p]; e < e1; e += 8) {
-    int j[8];
-    float y[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) j[q] = e + q < e1 ? col[e + q] : p;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) y[q] = x[j[q]];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) y[q] = normed(y[q], m, r);
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (e + q < e1) l = __fsub_rn(l, y[q]);
+struct PowerArgs {
+  int n, K, iterations;  // positions, chunks
+  const int32_t *ck_beg, *ck_end, *cl_ck, *beg, *end, *rp, *col, *clp;
+  const float *deg;
+  float *x, *y, *v;  // start vector in x; the last normalised vector goes to v
+  double *part;      // [3K]
+  unsigned int *sync;
+};
+
+__global__ void __launch_bounds__(kPowerThreads)
+part_power_kernel(PowerArgs a) {
+  extern __shared__ __align__(16) float power_sm[];
+  float *buf = power_sm;  // [kPowerEdges]: a chunk, chunk sums or neighbours
+  int32_t *col_s = reinterpret_cast<int32_t *>(power_sm + kPowerEdges);  // [kPowerEdges]
+  __shared__ float mean_s[kPowerClusters], nrm_s[kPowerClusters];
+  __shared__ int ca_s, cb_s;
+  __shared__ int range[2];
+  double *ps = reinterpret_cast<double *>(buf);
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  if (t == 0) {
+    ca_s = INT_MAX;
+    cb_s = -1;
   }
-  lv[p] = l;
+  // the block's positions: an even share of kPowerPos per position and one
+  // per neighbour
+  if (w < 2) {
+    const long long all = (long long)kPowerPos * a.n + a.rp[a.n];
+    const long long want = all * (blockIdx.x + w) / gridDim.x;
+    int lo = 0, hi = a.n;  // the first p with kPowerPos * p + rp[p] >= want lies in [lo, hi]
+    while (lo < hi) {      // 32 places a round, the last one short of hi
+      const int step = (hi - lo + 31) / 32, p = min(hi - 1, lo + lane * step);
+      const int below = __popc(__ballot_sync(
+          0xffffffffu, (long long)kPowerPos * p + a.rp[p] < want));
+      // places 0 .. below - 1 are too low
+      const int last = below ? min(hi - 1, lo + (below - 1) * step) : lo;
+      hi = below < 32 ? min(hi - 1, lo + below * step) : hi;
+      lo = below ? last + 1 : lo;
+    }
+    if (lane == 0) range[w] = lo;
+  }
+  __syncthreads();
+  const int p0 = range[0], p1 = range[1];
+  for (int p = p0 + t; p < p1; p += kPowerThreads) {
+    const int c = a.clp[p];
+    if (c >= 0) {
+      atomicMin(&ca_s, c);
+      atomicMax(&cb_s, c);
+    }
+  }
+  __syncthreads();
+  const int ca = ca_s, cb = cb_s;
+  const int kb = cb >= 0 ? a.cl_ck[ca] : 0, ke = cb >= 0 ? a.cl_ck[cb + 1] : 0;
+  // all neighbours at hand in one go, their positions kept in shared memory
+  const int r0 = a.rp[p0], edges = a.rp[p1] - r0;
+  const bool fits = edges <= kPowerEdges;
+  if (fits)
+    for (int i = t; i < edges; i += kPowerThreads) col_s[i] = a.col[r0 + i];
+  float *x = a.x, *y = a.y;
+  unsigned int target = 0;
+  for (int it = 0;; ++it) {
+    // chunk sums: the chunk in one round of loads, then warp 0 sums x, warp 1 x^2
+    for (int k = blockIdx.x; k < a.K; k += gridDim.x) {
+      const int b = a.ck_beg[k], m = a.ck_end[k] - b;
+      float u[kPartChunk / kPowerThreads];
+#pragma unroll
+      for (int r = 0; r < kPartChunk / kPowerThreads; ++r) {
+        const int i = r * kPowerThreads + t;
+        u[r] = i < m ? x[b + i] : 0.f;
+      }
+#pragma unroll
+      for (int r = 0; r < kPartChunk / kPowerThreads; ++r) ps[r * kPowerThreads + t] = (double)u[r];
+      __syncthreads();
+      if (w < 2) {
+        double s = 0.0;
+        if (w == 0) {
+#pragma unroll 16
+          for (int i = lane; i < m; i += 32) s += ps[i];
+        } else {
+#pragma unroll 16
+          for (int i = lane; i < m; i += 32) s += ps[i] * ps[i];
+        }
+        s = tree_sum(s);
+        if (lane == 0) a.part[3 * k + w] = s;
+      }
+      __syncthreads();
+    }
+    target += gridDim.x;
+    if (!all_meet(a.sync, target)) return;
+    // mean and norm of the block's clusters, chunks added in order
+    double s1[kPowerClusters / kPowerThreads] = {}, s2[kPowerClusters / kPowerThreads] = {};
+    for (int k0 = kb; k0 < ke; k0 += kPowerTile) {
+      const int k1 = min(ke, k0 + kPowerTile);
+      for (int i = t; i < 2 * (k1 - k0); i += kPowerThreads)
+        ps[i] = __ldcg(a.part + 3 * (size_t)(k0 + (i >> 1)) + (i & 1));
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kPowerClusters / kPowerThreads; ++r) {
+        const int c = ca + r * kPowerThreads + t;
+        if (c > cb) continue;
+        const int q1 = min(k1, a.cl_ck[c + 1]);
+#pragma unroll 4
+        for (int q = max(k0, a.cl_ck[c]); q < q1; ++q) {
+          s1[r] += ps[2 * (q - k0)];
+          s2[r] += ps[2 * (q - k0) + 1];
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < kPowerClusters / kPowerThreads; ++r) {
+      const int i = r * kPowerThreads + t, c = ca + i;
+      if (c <= cb)
+        mean_norm(s1[r], s2[r], (double)(a.end[c] - a.beg[c]), it > 0, mean_s[i], nrm_s[i]);
+    }
+    __syncthreads();
+    if (it == a.iterations) break;
+    // y = L normed(x), in the order of part_spmv_csr_kernel: neighbours are
+    // gathered and normalised edge by edge, then each position subtracts its
+    // row; all of the block's at once where they fit, else those of
+    // kPowerThreads positions a round, kPowerEdges at a time
+    auto gather = [&](const int32_t *col, int t0, int t1, int &ec, int &ec_end) {
+      for (int e = t0 + t; e < t1; e += 8 * kPowerThreads) {
+        float g[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int f = e + q * kPowerThreads;
+          g[q] = f < t1 ? x[col[f - t0]] : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int f = e + q * kPowerThreads;
+          if (f >= t1) break;
+          while (f >= ec_end) ec_end = a.rp[a.end[++ec]];
+          buf[f - t0] = normed(g[q], mean_s[ec - ca], nrm_s[ec - ca]);
+        }
+      }
+    };
+    auto subtract = [&](float l, const float *row, int m) {
+      for (int f = 0; f < m; f += 8) {
+        float g[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) g[q] = row[min(f + q, m - 1)];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (f + q < m) l = __fsub_rn(l, g[q]);
+      }
+      return l;
+    };
+    int ec = ca, ec_end = cb >= 0 ? a.rp[a.end[ca]] : 0;  // cluster of the edge at hand
+    if (fits) {
+      int p = p0 + t, c = -1, e0 = 0, e1 = 0;
+      float d = 0.f, xp = 0.f;
+      auto load = [&] {
+        if (p >= p1) return;
+        c = a.clp[p], e0 = a.rp[p], e1 = a.rp[p + 1], d = a.deg[p], xp = x[p];
+      };
+      load();
+      gather(col_s, r0, r0 + edges, ec, ec_end);
+      __syncthreads();
+      for (; p < p1; p += kPowerThreads, load()) {
+        if (c < 0) continue;
+        const float l = __fmul_rn(d, normed(xp, mean_s[c - ca], nrm_s[c - ca]));
+        y[p] = subtract(l, buf + (e0 - r0), e1 - e0);
+      }
+    } else {
+      for (int b0 = p0; b0 < p1; b0 += kPowerThreads) {
+        const int p = b0 + t, b1 = min(p1, b0 + kPowerThreads);
+        const int c = p < p1 ? a.clp[p] : -1;
+        const int e0 = p < p1 ? a.rp[p] : 0, e1 = p < p1 ? a.rp[p + 1] : 0;
+        float l = 0.f;
+        if (c >= 0) l = __fmul_rn(a.deg[p], normed(x[p], mean_s[c - ca], nrm_s[c - ca]));
+        const int te = a.rp[b1];
+        for (int t0 = a.rp[b0]; t0 < te; t0 += kPowerEdges) {
+          const int t1 = min(te, t0 + kPowerEdges);
+          gather(a.col + t0, t0, t1, ec, ec_end);
+          __syncthreads();
+          const int f0 = max(e0, t0), f1 = min(e1, t1);
+          if (f0 < f1) l = subtract(l, buf + (f0 - t0), f1 - f0);
+          __syncthreads();
+        }
+        if (c >= 0) y[p] = l;
+      }
+    }
+    target += gridDim.x;
+    if (!all_meet(a.sync, target)) return;
+    float *o = x;
+    x = y;
+    y = o;
+  }
+  for (int p = p0 + t; p < p1; p += kPowerThreads) {
+    const int c = a.clp[p];
+    if (c >= 0) a.v[p] = normed(x[p], mean_s[c - ca], nrm_s[c - ca]);
+  }
 }
 
 // ---- a whole depth of clusters of one chunk each --------------------------------
@@ -841,11 +983,11 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
     DevBuf<uint32_t> keys[2], th, ts, dt;
     DevBuf<int32_t> vals[2], slot_pos;
     DevBuf<float> lv2;
-    DevBuf<unsigned int> counters;         // last-block counter, CSR entries
+    DevBuf<unsigned int> counters;         // block arrivals, gave up; CSR entries
     DevBuf<unsigned long long> small_its;  // iterations of the one-chunk depths
-    FX_TRY(counters.alloc(2));
+    FX_TRY(counters.alloc(3));
     FX_TRY(small_its.alloc(1));
-    FX_CHECK_CUDA(cudaMemsetAsync(counters.p, 0, 8, s));
+    FX_CHECK_CUDA(cudaMemsetAsync(counters.p, 0, 12, s));
     FX_CHECK_CUDA(cudaMemsetAsync(small_its.p, 0, 8, s));
     FX_TRY(clp.alloc(N));
     FX_TRY(clg.alloc(N));
@@ -891,11 +1033,11 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
         const size_t smem = part_small_smem(most);
         const int threads = std::min(1024, std::max(96, (most / 2 + 31) / 32 * 32));
         FX_TRY(raise_smem_limit((const void *)part_small_kernel, (int)smem));
-        FX_CHECK_CUDA(cudaMemsetAsync(counters.p + 1, 0, 4, s));
+        FX_CHECK_CUDA(cudaMemsetAsync(counters.p + 2, 0, 4, s));
         part_small_kernel<<<C, threads, smem, s>>>(
             beg.p, end.p, most, d->adj_ptr.p, d->adj_idx.p, d_sin.p, cfg->power_iterations,
             cfg->tol, perm[cur].p, pos_of.p, reinterpret_cast<uint16_t *>(col.p),
-            counters.p + 1, small_its.p);
+            counters.p + 2, small_its.p);
         FX_CHECK_LAUNCH();
         ctx->launches += 1;
         FX_CHECK_CUDA(cudaStreamSynchronize(s));  // beg and end are reused
@@ -937,26 +1079,33 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       part_csr_kernel<<<nb, 256, 0, s>>>(N, perm[cur].p, pos_of.p, d->adj_ptr.p, d->adj_idx.p,
                                          clp.p, clg.p, rp.p, col.p);
       ctx->launches += 4;
-      const bool fixed = !exact && cfg->tol <= 0.0;
+      // a fixed count in one launch, where a block's positions span few enough
+      // clusters (clusters of a depth differ by one position, so up to 1e8 gates)
+      int least = N, per_sm = 0;
+      for (int c = 0; c < C; ++c) least = std::min(least, he[c] - hb[c]);
+      FX_TRY(raise_smem_limit((const void *)part_power_kernel, kPowerSmem));
+      FX_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, part_power_kernel,
+                                                                  kPowerThreads, kPowerSmem));
+      // blocks an SM so that a block's share fits its shared memory, if it can
+      const int64_t work = (int64_t)kPowerPos * N + d->a;
+      const int64_t share = (int64_t)ctx->num_sms * (kPowerEdges - kPowerEdges / 8);
+      const int grid = ctx->num_sms * (int)std::min<int64_t>(per_sm, (work + share - 1) / share);
+      // positions of a block: its share, all positions without neighbours
+      const int64_t per = grid > 0 ? ((int64_t)N + d->a / kPowerPos) / grid + 2 : N;
+      const bool fixed = !exact && cfg->tol <= 0.0 && grid > 0 && per / least + 2 <= kPowerClusters;
       if (fixed) {
-        // v holds the start vector; iterate x -> v = normed(x), lv = L v
         FX_TRY(lv2.alloc(N));
-        float *x = lv2.p, *y = lv.p;
-        FX_CHECK_CUDA(cudaMemcpyAsync(x, v.p, (size_t)N * 4, cudaMemcpyDeviceToDevice, s));
-        auto sums = [&](int deflate) {
-          part_sums_kernel<<<K, kSumThreads, 0, s>>>(C, ck_beg.p, ck_end.p, cl_ck.p, beg.p, end.p, x,
-                                            deflate, part.p, counters.p, mean.p, nrm.p);
-        };
-        sums(0);
-        for (int it = 0; it < cfg->power_iterations; ++it) {
-          part_step_kernel<<<nb, 256, 0, s>>>(N, rp.p, col.p, clp.p, deg.p, mean.p, nrm.p, x, v.p,
-                                              y);
-          std::swap(x, y);
-          sums(1);
-        }
-        part_div_kernel<<<nb, 256, 0, s>>>(N, clp.p, act.p, x, mean.p, nrm.p, v.p);
+        // the start vector is in v: x = v, and v gets the last one
+        FX_CHECK_CUDA(cudaMemcpyAsync(lv2.p, v.p, (size_t)N * 4, cudaMemcpyDeviceToDevice, s));
+        FX_CHECK_CUDA(cudaMemsetAsync(counters.p, 0, 4, s));
+        PowerArgs pa{N,     K,     cfg->power_iterations, ck_beg.p, ck_end.p, cl_ck.p,
+                     beg.p, end.p, rp.p,                  col.p,    clp.p,    deg.p,
+                     lv2.p, lv.p,  v.p,                   part.p,   counters.p};
+        void *args[] = {&pa};
+        FX_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)part_power_kernel, dim3(grid),
+                                                  dim3(kPowerThreads), args, kPowerSmem, s));
         FX_CHECK_LAUNCH();
-        ctx->launches += 2 + 2 * cfg->power_iterations;
+        ctx->launches += 1;
         total_iters += (int64_t)cfg->power_iterations * C;
       }
       // normalise the start vector (:151-156)
@@ -1041,8 +1190,14 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       FX_CHECK_CUDA(cudaStreamSynchronize(s));
     }
     unsigned long long si = 0;
+    unsigned int gave_up = 0;
     FX_CHECK_CUDA(cudaMemcpyAsync(&si, small_its.p, 8, cudaMemcpyDeviceToHost, s));
+    FX_CHECK_CUDA(cudaMemcpyAsync(&gave_up, counters.p + 1, 4, cudaMemcpyDeviceToHost, s));
     FX_CHECK_CUDA(cudaStreamSynchronize(s));
+    if (gave_up) {
+      set_error("fx_partition: a block waited too long for the others");
+      return FX_ECUDA;
+    }
     total_iters += (int64_t)si;
   }
   // outputs: leaves in position order, with their regions
