@@ -171,10 +171,10 @@ NCU_WALK = {
     "exact": {"dram": 61_725_696, "inst": 1_390_529_927, "tpi": 20.07,
               "limiter": "instruction issue: 87% issue-active, 0.5% of DRAM peak, "
                          "82% warps active"},
-    # bh_batch_walk_kernel<64, false>: 59.529 MB read + 1.481 MB written
-    "fast": {"dram": 61_009_920, "inst": 587_039_746, "tpi": 31.77,
-             "limiter": "instruction issue: 83% issue-active (ALU pipe 66%, FMA 33%), "
-                        "1.1% of DRAM peak, 52% warps active"},
+    # bh_batch_walk_kernel<64, false>: 59.6 MB read + 3.27 MB written
+    "fast": {"dram": 62_870_000, "inst": 425_900_000, "tpi": 31.8,
+             "limiter": "instruction issue: 75% issue-active (ALU pipe 59%, FMA 23%), "
+                        "1.4% of DRAM peak, 45% warps active"},
 }
 
 
@@ -227,6 +227,22 @@ def algorithmic(n, m, p, a, G, gc):
 
 
 # ---------------------------------------------------------------------------
+def cpu_barnes_hut(orc, x, y, threads, stride):
+    """Every stride-th point's forces by the reference's BarnesHutTree.cpp;
+    all points' by the oracle's restatement where the reference's sources are
+    not there to build it (cpu_bh_name says which)."""
+    bh = orc.bh_reference(x, y, 0.5, 0.5, 0.1, threads, stride=stride)
+    if bh is None:
+        r = orc.bh_forces(x, y, 0.5, 0.5, 0.1, threads)
+        bh = r["fx"], r["fy"]
+    return bh
+
+
+def cpu_bh_name(orc):
+    return ("the reference BarnesHutTree.cpp" if orc.ref_lib() is not None else
+            "a restatement of the Barnes-Hut walk (the reference's source is not here to build)")
+
+
 def cpu_iteration_sample(syn, x, y, bins, cong, threads, bh_stride, cong_stride):
     """Seconds per plain iteration of the CPU path, from a bounded sample.
 
@@ -244,12 +260,16 @@ def cpu_iteration_sample(syn, x, y, bins, cong, threads, bh_stride, cong_stride)
     fa = orc.attraction_f32(ap, ai, x, y, 1.0)
     t["attraction"] = time.perf_counter() - t0
     t0 = time.perf_counter()
-    orc.bh_reference(x, y, 0.5, 0.5, 0.1, threads, stride=len(x))
-    t_build = time.perf_counter() - t0
-    t0 = time.perf_counter()
-    bh = orc.bh_reference(x, y, 0.5, 0.5, 0.1, threads, stride=bh_stride)
-    t_samp = time.perf_counter() - t0
-    t["barnes_hut"] = t_build + max(t_samp - t_build, 0.0) * bh_stride
+    if orc.ref_lib() is None:
+        bh = cpu_barnes_hut(orc, x, y, threads, 1)
+        t["barnes_hut"] = time.perf_counter() - t0
+    else:
+        cpu_barnes_hut(orc, x, y, threads, len(x))
+        t_build = time.perf_counter() - t0
+        t0 = time.perf_counter()
+        bh = cpu_barnes_hut(orc, x, y, threads, bh_stride)
+        t_samp = time.perf_counter() - t0
+        t["barnes_hut"] = t_build + max(t_samp - t_build, 0.0) * bh_stride
     t0 = time.perf_counter()
     dens = orc.density_forces(x, y, area, c.chip_width, c.chip_height, bins, 0.7, 1e-4)
     t["density"] = time.perf_counter() - t0
@@ -308,7 +328,7 @@ def cpu_iteration_full(orc, s, adj, x, y, bins, cong, threads, sample=1):
     fa = orc.attraction_f32(ap, ai, x, y, 1.0)
     t["attraction"] = time.perf_counter() - t0
     t0 = time.perf_counter()
-    bh = orc.bh_reference(x, y, 0.5, 0.5, 0.1, threads, stride=sample)
+    bh = cpu_barnes_hut(orc, x, y, threads, sample)
     t["barnes_hut"] = time.perf_counter() - t0
     t0 = time.perf_counter()
     dens = orc.density_forces(x, y, area, s.chip_width, s.chip_height, bins, 0.7, 1e-4)
@@ -363,8 +383,8 @@ def run_reference(args, rank, world):
     sec = wall / args.steps
     value = 1.0 / sec
     sample = (f"{args.steps} full plain iterations on {args.gates} gates from the seeded start "
-              f"positions, every stage unsampled: attraction (1 thread), the reference "
-              f"BarnesHutTree.cpp (sequential build, walk on {threads} threads), the scipy DCT "
+              f"positions, every stage unsampled: attraction (1 thread), {cpu_bh_name(orc)} "
+              f"(sequential build, walk on {threads} threads), the scipy DCT "
               f"solve, the damped step, the literal congestion loops over all nets on "
               f"{threads} threads, HPWL")
     out = {"metric": METRIC, "value": value, "unit": UNIT, "impl": "reference",
@@ -582,8 +602,8 @@ def run_fluxion(args, rank, world, local_rank):
         cpu = {"value": 1.0 / sec, "unit": UNIT, "cores": 1, "kind": "port",
                "sample": "one plain iteration at the timed steps' start positions on 1 core: "
                          "attraction/integrate/HPWL (oracle restatement) and scipy DCT in "
-                         "full; reference BarnesHutTree.cpp walk of every 16th point and "
-                         "congestion of every 256th net, scaled",
+                         f"full; {cpu_bh_name(orc)} (the reference's: every 16th point, "
+                         "scaled) and congestion of every 256th net, scaled",
                "stage_seconds": {k: round(v, 4) for k, v in parts.items()}}
 
     out = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
