@@ -171,8 +171,8 @@ NCU_WALK = {
     "exact": {"dram": 61_725_696, "inst": 1_390_529_927, "tpi": 20.07,
               "limiter": "instruction issue: 87% issue-active, 0.5% of DRAM peak, "
                          "82% warps active"},
-    # bh_batch_walk_kernel<64, false>: 59.6 MB read + 3.27 MB written
-    "fast": {"dram": 62_870_000, "inst": 425_900_000, "tpi": 31.8,
+    # bh_batch_walk_kernel<64, false>: 59.504 MB read + 2.190 MB written
+    "fast": {"dram": 61_693_952, "inst": 426_078_402, "tpi": 28.94,
              "limiter": "instruction issue: 75% issue-active (ALU pipe 59%, FMA 23%), "
                         "1.4% of DRAM peak, 45% warps active"},
 }
@@ -901,15 +901,9 @@ def run_leaves(args, rank, world, local_rank):
     lg = np.arange(c.num_gates, dtype=np.int32)
     sizes = np.diff(lp).astype(np.int64)
     pairs = int((sizes * (sizes - 1) // 2).sum())
-    # the call uploads the caller's lists and positions plus what it derives:
-    # the in-leaf adjacency (row offsets, int16 neighbour slots) and the order
-    ap_all, ai_all = fx.build_adjacency(c)
-    leaf_of = np.empty(c.num_gates, np.int64)
-    leaf_of[lg] = np.repeat(np.arange(len(sizes)), sizes)
-    in_leaf = int((leaf_of[np.repeat(np.arange(c.num_gates), np.diff(ap_all))]
-                   == leaf_of[ai_all]).sum())
+    # the call uploads the caller's lists and positions and the processing order
     h2d_bytes = (4 * (len(lp) + c.num_gates) + 16 * args.clusters + 8 * c.num_gates
-                 + 4 * (c.num_gates + 1) + 2 * in_leaf + 4 * args.clusters)
+                 + 4 * args.clusters)
     ctx = fx.Context(local_rank)
     d = fx.Design(ctx, c)
     fast = args.leaf_precision == "fast"
@@ -988,8 +982,7 @@ def run_leaves(args, rank, world, local_rank):
            "e2e": {"value": world * units * args.steps / wall, "unit": "cluster-iterations/s",
                    "h2d_bytes_per_step": h2d_bytes,
                    "d2h_bytes_per_step": 8 * c.num_gates,
-                   "call": "fx_hapr_place_leaves with host leaf lists and regions (the "
-                           "in-leaf adjacency it derives on the host is uploaded too)"},
+                   "call": "fx_hapr_place_leaves with host leaf lists and regions"},
            "gpu_launches": launches, "clocks": clk}
     if rank == 0:
         print(json.dumps(out), flush=True)
@@ -1095,11 +1088,11 @@ def run_precision(args, rank, world, local_rank):
     out = {"metric": PREC_METRIC, "value": best["tensor_tflops_executed"], "unit": "TFLOP/s",
            "n_gpus": 1, "steps": 3, "warmup": 1, "ms_per_step": best["density_ms"],
            "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-           "dtype": "bf16/tf32/3xtf32/fp32 (FP32 accumulate), int8 slices (int32 accumulate)",
+           "dtype": "bf16/tf32/3xtf32 (FP32 accumulate), fp32 (fast DCT, FP64 arithmetic)",
            "data": "synthetic",
            "config": {"workload": f"precision: {n} gates, die 2400, G in (2048, 4096), "
                                   "target density 0.7, weight 1", "seed": args.seed,
-                      "peak_source": f"{src} bf16 dense (tf32: half, int8: twice)"},
+                      "peak_source": f"{src} bf16 dense (tf32: half)"},
            "value_is": f"{best['precision']} at G=4096, executed tensor FLOP/s of the 6 GEMMs",
            "sweep": rows}
     print(json.dumps(out), flush=True)

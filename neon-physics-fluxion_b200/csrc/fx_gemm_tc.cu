@@ -313,8 +313,8 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// A rows x cols row-major operand of esz-byte elements (4: f32, 2: bf16,
-// 1: int8 slices) as a 2-D tensor map with 128 x 128-byte boxes.
+// A rows x cols row-major operand of esz-byte elements (4: f32, 2: bf16)
+// as a 2-D tensor map with 128 x 128-byte boxes.
 static int make_map(const void *ptr, int cols, int rows, int esz, CUtensorMap *out,
                     int box_rows = 128) {
   EncodeTiledFn fn = encode_fn();
@@ -332,9 +332,7 @@ static int make_map(const void *ptr, int cols, int rows, int esz, CUtensorMap *o
   const cuuint32_t estr[2] = {1u, 1u};
   const CUresult r =
       fn(out,
-         esz == 1   ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-         : esz == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                    : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+         esz == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
          2,
          const_cast<void *>(ptr), dims, strides, box, estr,
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
