@@ -174,7 +174,8 @@ __global__ void part_csr_kernel(int n, const int32_t *__restrict__ perm,
                                 const int32_t *__restrict__ adj_ptr,
                                 const int32_t *__restrict__ adj_idx,
                                 const int32_t *__restrict__ clp,
-                                const int32_t *__restrict__ clg,
+                                const int32_t *__restrict__ beg,
+                                const int32_t *__restrict__ end,
                                 const int32_t *__restrict__ rp, int32_t *__restrict__ col) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
@@ -182,9 +183,11 @@ __global__ void part_csr_kernel(int n, const int32_t *__restrict__ perm,
   if (c < 0) return;
   const int g = perm[p];
   int k = rp[p];
-  for (int e = adj_ptr[g]; e < adj_ptr[g + 1]; ++e) {
-    const int j = adj_idx[e];
-    if (clg[j] == c) col[k++] = pos_of[j];
+  // a cluster is a segment of positions
+  const int b = beg[c], e = end[c];
+  for (int q = adj_ptr[g], q1 = adj_ptr[g + 1]; q < q1; ++q) {
+    const int t = pos_of[adj_idx[q]];
+    if (t >= b && t < e) col[k++] = t;
   }
 }
 
@@ -393,7 +396,7 @@ __global__ void part_combine_kernel(int C, const int32_t *__restrict__ beg,
 // 128 dependent FP64 sums. Blocks get even shares of positions and neighbours,
 // not of positions: the order by Fiedler value gathers the hubs at the ends
 // (9.9 us a product by positions, 4.3 by shares). A hierarchy of 100k gates
-// takes 3.7 ms (5.4 before), of 1M 17.2.
+// takes 3.6 ms (5.4 before), of 1M 16.9.
 constexpr int kPowerThreads = 512;
 constexpr int kPowerClusters = 1024;      // clusters the positions of a block may span
 constexpr int kPowerTile = kPartChunk / 4;  // chunk sums staged at a time
@@ -617,12 +620,31 @@ part_power_kernel(PowerArgs a) {
   }
 }
 
+// take(map[idx[q]]) for q in [q0, q1) in order, 16 entries' loads in flight:
+// the longest rows (129 neighbours at 100k gates) set the time of a block's
+// row passes, two L2 round trips a batch (a depth 134 -> 127 us).
+template <class F>
+__device__ __forceinline__ void each_neighbour(const int32_t *__restrict__ idx, int q0, int q1,
+                                               const int32_t *map, F take) {
+  for (int q = q0; q < q1; q += 16) {
+    int32_t j[16], m[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) j[u] = idx[min(q + u, q1 - 1)];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) m[u] = map[j[u]];
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      if (q + u < q1) take(m[u]);
+  }
+}
+
 // ---- a whole depth of clusters of one chunk each --------------------------------
 // A block per cluster of at most kPartChunk positions does all that the depth
 // does to it: the in-cluster CSR, every power iteration with the vectors in
 // shared memory, the stable sort by Fiedler value (position breaks ties, so
 // a bitonic sort of (key, place) pairs is stable) and the new order. One
-// launch of 141 us (a depth of 100k gates, ncu cold) instead of 4 * 30 + 25
+// launch of 127 us (a depth of 100k gates, ncu cold; 141 with a warp per sum
+// and mean and norm in every thread) instead of 4 * 30 + 25
 // launches of 1.2 ms: the lower depths' clusters of some hundred gates left
 // each launch waiting on one chain of sums. Bound by that chain (a lane's 128
 // dependent FP64 sums) and the barriers of 30 iterations. The sums keep the
@@ -651,14 +673,17 @@ part_small_kernel(const int32_t *__restrict__ beg, const int32_t *__restrict__ e
   int32_t *rp = reinterpret_cast<int32_t *>(lv + most);
   __shared__ int32_t wsum[32];
   __shared__ unsigned int base_sh;
-  __shared__ double sums[3];
+  __shared__ double lambda_sh;
+  __shared__ float mean_sh, nrm_sh;
+  double *ld = reinterpret_cast<double *>(key);  // lv in FP64; the keys come after the iterations
   const int T = blockDim.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int b = beg[blockIdx.x], e = end[blockIdx.x], n = e - b;
   // in-cluster CSR: counts, row starts, columns (local places)
   for (int i = t; i < n; i += T) {
     const int g = perm[b + i], q1 = adj_ptr[g + 1];
     int c = 0;
-    for (int q = adj_ptr[g]; q < q1; ++q) c += (unsigned)(pos_of[adj_idx[q]] - b) < (unsigned)n;
+    each_neighbour(adj_idx, adj_ptr[g], q1, pos_of,
+                   [&](int p) { c += (unsigned)(p - b) < (unsigned)n; });
     rp[i + 1] = c;
   }
   __syncthreads();
@@ -687,43 +712,43 @@ part_small_kernel(const int32_t *__restrict__ beg, const int32_t *__restrict__ e
   for (int i = t; i < n; i += T) {
     const int g = perm[b + i], q1 = adj_ptr[g + 1];
     int k = rp[i];
-    for (int q = adj_ptr[g]; q < q1; ++q) {
-      const int r = pos_of[adj_idx[q]] - b;
-      if ((unsigned)r < (unsigned)n) mine[k++] = (uint16_t)r;
-    }
+    each_neighbour(adj_idx, adj_ptr[g], q1, pos_of, [&](int p) {
+      if ((unsigned)(p - b) < (unsigned)n) mine[k++] = (uint16_t)(p - b);
+    });
     lv[i] = sin_tab[i];
+    ld[i] = (double)lv[i];
   }
   __syncthreads();
-  // sums over x = lv (and v), one kind per warp; then v = normed(lv)
-  auto reduce = [&](bool with_v) {
-    if (w < 2 || (w == 2 && with_v)) {
-      double s = 0.0;
-      if (w == 0) {
-#pragma unroll 8
-        for (int i = lane; i < n; i += 32) s += (double)lv[i];
-      } else if (w == 1) {
-#pragma unroll 8
-        for (int i = lane; i < n; i += 32) {
-          const double a = (double)lv[i];
-          s += a * a;
-        }
-      } else {
-#pragma unroll 8
-        for (int i = lane; i < n; i += 32) s += (double)v[i] * (double)lv[i];
+  // warp 0 sums x = lv and x^2 (two chains at once, from FP64 copies) and
+  // has mean and norm; warp 1 sums v.x where the stop test asks for it
+  auto reduce = [&](int deflate) {
+    if (w == 0) {
+      double s1 = 0.0, s2 = 0.0;
+#pragma unroll 16
+      for (int i = lane; i < n; i += 32) {
+        const double a = ld[i];
+        s1 += a;
+        s2 += a * a;
       }
+      s1 = tree_sum(s1);
+      s2 = tree_sum(s2);
+      if (lane == 0) mean_norm(0.0 + s1, 0.0 + s2, (double)n, deflate, mean_sh, nrm_sh);
+    } else if (w == 1 && deflate && tol > 0.0) {
+      double s = 0.0;
+#pragma unroll 8
+      for (int i = lane; i < n; i += 32) s += (double)v[i] * ld[i];
       s = tree_sum(s);
-      if (lane == 0) sums[w] = 0.0 + s;
+      if (lane == 0) lambda_sh = 0.0 + s;
     }
     __syncthreads();
   };
-  auto normalise = [&](int deflate) {
-    float m, r;
-    mean_norm(sums[0], sums[1], (double)n, deflate, m, r);
+  auto normalise = [&] {
+    const float m = mean_sh, r = nrm_sh;
     for (int i = t; i < n; i += T) v[i] = normed(lv[i], m, r);
     __syncthreads();
   };
-  reduce(false);
-  normalise(0);
+  reduce(0);
+  normalise();
   double lambda = 0.0;
   int it = 0;
   while (it < iterations) {
@@ -739,14 +764,15 @@ part_small_kernel(const int32_t *__restrict__ beg, const int32_t *__restrict__ e
           if (k + q < k1) l = __fsub_rn(l, v[j[q]]);
       }
       lv[i] = l;
+      ld[i] = (double)l;
     }
     __syncthreads();
-    reduce(true);
+    reduce(1);
     ++it;
     const double prev = lambda;
-    lambda = sums[2];
+    if (tol > 0.0) lambda = lambda_sh;
     const bool stop = tol > 0.0 && it > 1 && fabs(lambda - prev) <= tol * fabs(lambda);
-    normalise(1);  // a converged cluster takes this update as its last
+    normalise();  // a converged cluster takes this update as its last
     if (stop) break;
   }
   if (t == 0 && it > 0) atomicAdd(iters, (unsigned long long)it);
@@ -1077,7 +1103,7 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       part_scan_top_kernel<<<1, 1024, 0, s>>>(st, tsum.p);
       part_scan_add_kernel<<<nb, 256, 0, s>>>(N, st, tsum.p, rp.p);
       part_csr_kernel<<<nb, 256, 0, s>>>(N, perm[cur].p, pos_of.p, d->adj_ptr.p, d->adj_idx.p,
-                                         clp.p, clg.p, rp.p, col.p);
+                                         clp.p, beg.p, end.p, rp.p, col.p);
       ctx->launches += 4;
       // a fixed count in one launch, where a block's positions span few enough
       // clusters (clusters of a depth differ by one position, so up to 1e8 gates)
