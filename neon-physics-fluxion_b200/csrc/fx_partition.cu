@@ -1118,7 +1118,7 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       const int grid = ctx->num_sms * (int)std::min<int64_t>(per_sm, (work + share - 1) / share);
       // positions of a block: its share, all positions without neighbours
       const int64_t per = grid > 0 ? ((int64_t)N + d->a / kPowerPos) / grid + 2 : N;
-      const bool fixed = !exact && cfg->tol <= 0.0 && grid > 0 && per / least + 2 <= kPowerClusters;
+      bool fixed = !exact && cfg->tol <= 0.0 && grid > 0 && per / least + 2 <= kPowerClusters;
       if (fixed) {
         FX_TRY(lv2.alloc(N));
         // the start vector is in v: x = v, and v gets the last one
@@ -1128,11 +1128,16 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
                      beg.p, end.p, rp.p,                  col.p,    clp.p,    deg.p,
                      lv2.p, lv.p,  v.p,                   part.p,   counters.p};
         void *args[] = {&pa};
-        FX_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)part_power_kernel, dim3(grid),
-                                                  dim3(kPowerThreads), args, kPowerSmem, s));
-        FX_CHECK_LAUNCH();
-        ctx->launches += 1;
-        total_iters += (int64_t)cfg->power_iterations * C;
+        const cudaError_t e = cudaLaunchCooperativeKernel((const void *)part_power_kernel, dim3(grid),
+                                                          dim3(kPowerThreads), args, kPowerSmem, s);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {  // a share of the device: step by step
+          cudaGetLastError();
+          fixed = false;
+        } else {
+          FX_CHECK_CUDA(e);
+          ctx->launches += 1;
+          total_iters += (int64_t)cfg->power_iterations * C;
+        }
       }
       // normalise the start vector (:151-156)
       if (fixed) {
