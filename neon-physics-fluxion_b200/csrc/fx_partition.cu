@@ -475,7 +475,9 @@ part_power_kernel(PowerArgs a) {
     }
   }
   __syncthreads();
-  const int ca = ca_s, cb = cb_s;
+  // A share can hold no cluster: positions of leaves only, or none at all
+  // beside a row longer than a share. Its range is then the empty [0, -1].
+  const int cb = cb_s, ca = cb >= 0 ? ca_s : 0;
   const int kb = cb >= 0 ? a.cl_ck[ca] : 0, ke = cb >= 0 ? a.cl_ck[cb + 1] : 0;
   // all neighbours at hand in one go, their positions kept in shared memory
   const int r0 = a.rp[p0], edges = a.rp[p1] - r0;
