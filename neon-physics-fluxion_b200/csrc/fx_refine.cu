@@ -52,15 +52,18 @@ constexpr int kTotalThreads = 512, kTotalItems = 8, kTotalWarps = kTotalThreads 
 constexpr int kTotalChunk = kTotalThreads * kTotalItems;
 constexpr int kTotalHead = 512;      // cells one lane folds first: the sum doubles often there
 constexpr int kTotalFull = 1 << 24;  // units where the binade ends
-// A term of 2^22 units or more counts as this many: it is added by itself.
+// A term of kTotalWhole units or more counts as kTotalSat: it is added by itself.
 constexpr int kTotalSat = 1 << 25;
+// Below this both additions of total_term are whole to the unit: the larger
+// one, to 1.5 * 2^23 + 1, stays below 2^24, where the spacing becomes 2.
+constexpr float kTotalWhole = 4194303.0f;
 
 // Increment of the sum for a term of t = a / u units (exact), as {from even
 // S, from odd S}: t rounded once to an integer, ties to the parity that makes
 // S plus it even, by one f32 addition to 1.5 * 2^23 or to the odd number after
 // it (no conversions, which run at an eighth of the addition rate).
 __device__ __forceinline__ int2 total_term(float t) {
-  if (!(t < 4194304.0f)) return make_int2(kTotalSat, kTotalSat);
+  if (!(t < kTotalWhole)) return make_int2(kTotalSat, kTotalSat);
   return make_int2(__float_as_int(__fadd_rn(t, 12582912.0f)) - 0x4b400000,
                    __float_as_int(__fadd_rn(t, 12582913.0f)) - 0x4b400001);
 }
