@@ -16,6 +16,7 @@ namespace fx {
 
 static thread_local char g_err[512] = "";
 thread_local cudaStream_t g_alloc_stream = nullptr;
+thread_local int g_fail_alloc = 0;
 
 void set_error(const char *fmt, ...) {
   va_list ap;
@@ -356,6 +357,15 @@ extern "C" int fx_ctx_reset_stage_times(fx_ctx *ctx) {
     ctx->timer.calls[s] = 0;
   }
   return FX_OK;
+}
+
+// A test setting, not part of the interface: the calling thread's nth device
+// allocation from here on fails as if the device were full (0: none does).
+// Returns what was left of the last count: 0 when that failure has happened.
+extern "C" int fx_test_fail_alloc(int nth) {
+  const int left = g_fail_alloc;
+  g_fail_alloc = nth;
+  return left;
 }
 
 extern "C" int64_t fx_ctx_kernel_launches(fx_ctx *ctx) {

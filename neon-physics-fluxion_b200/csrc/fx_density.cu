@@ -222,6 +222,9 @@ static int dens_setup_fast(fx_design *d, int G, int precision, cudaStream_t s) {
 static int dens_setup(fx_design *d, int G, int precision, cudaStream_t s) {
   DensityWork &w = d->dens;
   if (w.G == G && w.precision == precision && w.area_fx.p) return FX_OK;
+  // the buffers' contents belong to no grid until the setup has run through: one
+  // that fails on the way must not leave the previous grid's key behind
+  w.G = 0;
   const size_t cells = (size_t)G * G;
   if (dct_fast(precision)) return dens_setup_fast(d, G, precision, s);
   FX_TRY(w.area_fx.alloc(cells));

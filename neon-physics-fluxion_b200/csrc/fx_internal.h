@@ -48,6 +48,9 @@ struct Status {
 // event recorded on it later. Without a scope (library globals) DevBuf uses
 // cudaMalloc / cudaFree.
 extern thread_local cudaStream_t g_alloc_stream;
+// Test setting (fx_test_fail_alloc): the calling thread's allocation with this
+// number, counted from 1, fails; 0: none does.
+extern thread_local int g_fail_alloc;
 
 struct AllocScope {
   cudaStream_t prev;
@@ -73,7 +76,9 @@ struct DevBuf {
     release();
     if (count == 0) return FX_OK;
     cudaError_t e;
-    if (g_alloc_stream) {
+    if (g_fail_alloc > 0 && --g_fail_alloc == 0) {
+      e = cudaErrorMemoryAllocation;
+    } else if (g_alloc_stream) {
       e = cudaMallocAsync((void **)&p, count * sizeof(T), g_alloc_stream);
       pooled = true;
       owner = g_alloc_stream;
