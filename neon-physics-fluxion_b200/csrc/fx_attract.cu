@@ -269,12 +269,11 @@ static int step_alloc(fx_design *d, cudaStream_t s) {
   StepWork &w = d->step;
   const size_t nb = ((size_t)d->n + kGates - 1) / kGates;
   if (w.e_part.p && w.e_part.n >= nb) return FX_OK;
-  FX_TRY(w.e_part.alloc(nb));
   FX_TRY(w.done.alloc(4));
   FX_TRY(w.energy.alloc(4));
   FX_CHECK_CUDA(cudaMemsetAsync(w.done.p, 0, 16, s));
   FX_CHECK_CUDA(cudaMemsetAsync(w.energy.p, 0, 32, s));
-  return FX_OK;
+  return w.e_part.alloc(nb);  // last: it stands for all of them
 }
 
 static int validate_cfg(const fx_iter_cfg &c) {

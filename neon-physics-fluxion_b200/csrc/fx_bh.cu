@@ -1601,7 +1601,7 @@ static int bh_alloc(fx_design *d) {
 static int bh_alloc_deep(fx_design *d) {
   BHWork &b = d->bh;
   const size_t n = (size_t)d->n;
-  if (b.klo.p && b.klo.n >= n) return FX_OK;
+  if (b.slo.p && b.slo.n >= n) return FX_OK;  // the last one
   FX_TRY(b.klo.alloc(n));
   FX_TRY(b.kl[0].alloc(n));
   FX_TRY(b.kl[1].alloc(n));

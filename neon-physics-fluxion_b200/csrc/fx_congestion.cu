@@ -241,6 +241,7 @@ int congestion_alloc(fx_design *d, int cols, int rows, cudaStream_t s) {
   }
   if (w.cols != cols || w.rows != rows || !w.diff.p) {
     const size_t cells1 = (size_t)(cols + 1) * (rows + 1);
+    w.cols = w.rows = 0;  // no grid's buffers until all are there and zeroed
     FX_TRY(w.diff.alloc(cells1));
     FX_TRY(w.counts.alloc((size_t)cols * rows));
     FX_TRY(w.partial.alloc(kMaxNetBlocks + 4096));

@@ -669,7 +669,7 @@ extern "C" int fx_design_save_state(fx_design *d) {
 
 extern "C" int fx_design_restore_state(fx_design *d) {
   if (!d) return FX_EINVAL;
-  if (!d->saved[0].p) {
+  if (!d->saved[3].p) {  // the last one: a save has run through
     set_error("fx_design_restore_state: no saved state");
     return FX_EINVAL;
   }
