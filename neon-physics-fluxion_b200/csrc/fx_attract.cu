@@ -22,6 +22,7 @@
 
 namespace fx {
 
+int bh_reserve(fx_design *d, float theta, float min_dist);
 int bh_bbox(fx_ctx *ctx, fx_design *d, const float *x, const float *y,
             cudaStream_t s);
 int density_prepare(fx_design *d, int G, int precision, cudaStream_t s);
@@ -427,20 +428,23 @@ extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
   const bool use_dens = c.density_bins > 0 && c.density_weight != 0.f;
   const bool use_cong = c.cong_cols > 0;
   const int G = c.density_bins;
+  // Every workspace, and the refusal of grids that none fits, before anything
+  // is launched and whatever the number of iterations.
+  if (use_dens) FX_TRY(density_prepare(d, G, c.dct_precision, s));
+  if (use_bh) FX_TRY(bh_reserve(d, c.theta, c.min_dist));
+  if (use_cong) FX_TRY(congestion_alloc(d, c.cong_cols, c.cong_rows, s));
   // Bounding box / density of the starting positions; each step then
   // prepares both for the positions it writes.
   auto prologue = [&]() -> int {
     // the scatter feeds the density solve alone, so it runs on the second
     // stream beside the box and the tree (the first step joins it)
     if (use_dens) {
-      FX_TRY(density_prepare(d, G, c.dct_precision, s));
       FX_CHECK_CUDA(cudaEventRecord(ctx->fork, s));
       FX_CHECK_CUDA(cudaStreamWaitEvent(s2, ctx->fork, 0));
       FX_TRY(density_scatter(ctx, d, d->x[d->cur].p, d->y[d->cur].p, G,
                              c.dct_precision, s2));
     }
     if (use_bh) FX_TRY(bh_bbox(ctx, d, d->x[d->cur].p, d->y[d->cur].p, s));
-    if (use_cong) FX_TRY(congestion_alloc(d, c.cong_cols, c.cong_rows, s));
     return FX_OK;
   };
   const int nb = (d->n + kGates - 1) / kGates;

@@ -1621,6 +1621,12 @@ static bool bh_maybe_deep(const fx_design *d, float th2, float md2) {
   return s15 * s15 >= (double)th2 * (double)md2 * (1.0 - 1e-6);
 }
 
+// All buffers of bh_run on the design's present positions.
+int bh_reserve(fx_design *d, float theta, float min_dist) {
+  FX_TRY(bh_alloc(d));
+  return bh_maybe_deep(d, theta * theta, min_dist * min_dist) ? bh_alloc_deep(d) : FX_OK;
+}
+
 // The walk's and the sort's error word (bh.bbox[4]) as a status.
 int bh_error(unsigned int err) {
   if (err & 4u) {

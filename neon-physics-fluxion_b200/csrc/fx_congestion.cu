@@ -239,6 +239,10 @@ int congestion_alloc(fx_design *d, int cols, int rows, cudaStream_t s) {
     set_error("congestion grid %d x %d too large", cols, rows);
     return FX_EINVAL;
   }
+  if ((cols + 31) / 32 > 4096) {  // the column scan's partial results
+    set_error("congestion grid too wide (%d columns)", cols);
+    return FX_EINVAL;
+  }
   if (w.cols != cols || w.rows != rows || !w.diff.p) {
     const size_t cells1 = (size_t)(cols + 1) * (rows + 1);
     w.cols = w.rows = 0;  // no grid's buffers until all are there and zeroed
@@ -276,11 +280,6 @@ int congestion_run(fx_ctx *ctx, fx_design *d, const float *dx,
   FX_CHECK_LAUNCH();
   cong_scan_rows_kernel<<<rows, 1024, 0, s>>>(w.diff.p, cols, rows);
   FX_CHECK_LAUNCH();
-  const int cb = (cols + 31) / 32;
-  if (cb > 4096) {
-    set_error("congestion grid too wide (%d columns)", cols);
-    return FX_EINVAL;
-  }
   launch_scan_cols(w.diff.p, w.counts.p, cols, rows, cap, w.partial.p + kMaxNetBlocks,
                    w.partial_max.p, w.done.p + 1, w.result.p, w.result_max.p, s);
   FX_CHECK_LAUNCH();
