@@ -409,13 +409,8 @@ static std::vector<uint64_t> iter_graph_key(fx_ctx *ctx, fx_design *d, const fx_
   return k;
 }
 
-extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
-                                const fx_iter_cfg *cfg, int32_t iters, float *x,
-                                float *y, fx_iter_stats *stats) {
-  if (!ctx || !d || !cfg || iters < 0 || (x == nullptr) != (y == nullptr)) {
-    set_error("fx_force_iterate: invalid arguments");
-    return FX_EINVAL;
-  }
+static int force_iterate(fx_ctx *ctx, fx_design *d, const fx_iter_cfg *cfg, int32_t iters,
+                         float *x, float *y, fx_iter_stats *stats) {
   const fx_iter_cfg c = *cfg;
   FX_TRY(validate_cfg(c));
   FX_CHECK_CUDA(cudaSetDevice(ctx->device));
@@ -662,14 +657,7 @@ extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
     }
     if (graph) cudaGraphDestroy(graph);
   }
-  for (; it < iters; ++it) {
-    const int rc = step(it == iters - 1);
-    if (rc != FX_OK) {
-      // never return while a copy into the caller's buffers is in flight
-      if (copied_out) cudaStreamSynchronize(s2);
-      return rc;
-    }
-  }
+  for (; it < iters; ++it) FX_TRY(step(it == iters - 1));
   fx_iter_stats st{};
   st.iterations = iters;
   // the statistics come back through the context's pinned buffer (truly
@@ -708,6 +696,21 @@ extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
   if (x && !copied_out) FX_TRY(fx_design_get_positions(d, x, y));
   if (stats) *stats = st;
   return FX_OK;
+}
+
+extern "C" int fx_force_iterate(fx_ctx *ctx, fx_design *d,
+                                const fx_iter_cfg *cfg, int32_t iters, float *x,
+                                float *y, fx_iter_stats *stats) {
+  if (!ctx || !d || !cfg || iters < 0 || (x == nullptr) != (y == nullptr)) {
+    set_error("fx_force_iterate: invalid arguments");
+    return FX_EINVAL;
+  }
+  const int rc = force_iterate(ctx, d, cfg, iters, x, y, stats);
+  // An error can leave the second stream's scatter, solve or congestion, which
+  // nothing has joined, or a copy into the caller's buffers in flight: later
+  // calls order their work on the primary stream alone.
+  if (rc != FX_OK) cudaStreamSynchronize(ctx->stream2);
+  return rc;
 }
 
 extern "C" int fx_design_trace(fx_design *d, int enable) {
