@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstdlib>
 #include <vector>
 
 #include "fx_internal.h"
@@ -406,10 +407,22 @@ constexpr int kPowerPos = 8;  // work of a position, in neighbours
 constexpr int kPowerSmem = 2 * kPowerEdges * 4;
 constexpr int kMeetSpin = 1 << 22;        // polls before a block gives up (seconds)
 
+// Polls a block may make at a meeting (kMeetSpin; less when the environment
+// variable FLUXION_PART_MEET_POLLS asks for it, a test setting that makes the
+// wait run out).
+int meet_polls() {
+  static const int polls = [] {
+    const char *e = std::getenv("FLUXION_PART_MEET_POLLS");
+    const int v = e ? std::atoi(e) : kMeetSpin;
+    return std::min(kMeetSpin, std::max(1, v));
+  }();
+  return polls;
+}
+
 // Every block arrives and waits for the others, which a cooperative launch
 // keeps resident; sync[0] counts arrivals (target: those so far and this
 // meeting's), sync[1] is set by a block that gave up. True if all went well.
-__device__ bool all_meet(unsigned int *sync, unsigned int target) {
+__device__ bool all_meet(unsigned int *sync, unsigned int target, int polls) {
   __syncthreads();
   bool bad = false;
   if (threadIdx.x == 0) {
@@ -418,15 +431,15 @@ __device__ bool all_meet(unsigned int *sync, unsigned int target) {
     unsigned int seen;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync) : "memory");
-    } while ((int)(seen - target) < 0 && ++spin < kMeetSpin);
-    bad = spin >= kMeetSpin;
+    } while ((int)(seen - target) < 0 && ++spin < polls);
+    bad = spin >= polls;
     if (bad) atomicExch(sync + 1, 1u);
   }
   return !__syncthreads_or(bad);
 }
 
 struct PowerArgs {
-  int n, K, iterations;  // positions, chunks
+  int n, K, iterations, polls;  // positions, chunks
   const int32_t *ck_beg, *ck_end, *cl_ck, *beg, *end, *rp, *col, *clp;
   const float *deg;
   float *x, *y, *v;  // start vector in x; the last normalised vector goes to v
@@ -514,7 +527,7 @@ part_power_kernel(PowerArgs a) {
       __syncthreads();
     }
     target += gridDim.x;
-    if (!all_meet(a.sync, target)) return;
+    if (!all_meet(a.sync, target, a.polls)) return;
     // mean and norm of the block's clusters, chunks added in order
     double s1[kPowerClusters / kPowerThreads] = {}, s2[kPowerClusters / kPowerThreads] = {};
     for (int k0 = kb; k0 < ke; k0 += kPowerTile) {
@@ -611,7 +624,7 @@ part_power_kernel(PowerArgs a) {
       }
     }
     target += gridDim.x;
-    if (!all_meet(a.sync, target)) return;
+    if (!all_meet(a.sync, target, a.polls)) return;
     float *o = x;
     x = y;
     y = o;
@@ -1126,9 +1139,10 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
         // the start vector is in v: x = v, and v gets the last one
         FX_CHECK_CUDA(cudaMemcpyAsync(lv2.p, v.p, (size_t)N * 4, cudaMemcpyDeviceToDevice, s));
         FX_CHECK_CUDA(cudaMemsetAsync(counters.p, 0, 4, s));
-        PowerArgs pa{N,     K,     cfg->power_iterations, ck_beg.p, ck_end.p, cl_ck.p,
-                     beg.p, end.p, rp.p,                  col.p,    clp.p,    deg.p,
-                     lv2.p, lv.p,  v.p,                   part.p,   counters.p};
+        PowerArgs pa{N,        K,        cfg->power_iterations, meet_polls(), ck_beg.p,
+                     ck_end.p, cl_ck.p,  beg.p,                 end.p,        rp.p,
+                     col.p,    clp.p,    deg.p,                 lv2.p,        lv.p,
+                     v.p,      part.p,   counters.p};
         void *args[] = {&pa};
         const cudaError_t e = cudaLaunchCooperativeKernel((const void *)part_power_kernel, dim3(grid),
                                                           dim3(kPowerThreads), args, kPowerSmem, s);
@@ -1228,8 +1242,8 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
     FX_CHECK_CUDA(cudaMemcpyAsync(&gave_up, counters.p + 1, 4, cudaMemcpyDeviceToHost, s));
     FX_CHECK_CUDA(cudaStreamSynchronize(s));
     if (gave_up) {
-      set_error("fx_partition: a block waited too long for the others");
-      return FX_ECUDA;
+      set_error("fx_partition: a bounded wait of a block for the others expired");
+      return FX_ETIMEOUT;
     }
     total_iters += (int64_t)si;
   }
