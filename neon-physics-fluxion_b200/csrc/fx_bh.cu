@@ -1740,9 +1740,9 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
   cudaEvent_t ev;
   int launches = 0;
   // Small designs: one cluster does keys and sort (fx_bh_sort.cu) up to its
-  // capacity: 20 us at 5k points and 28 at 10k against 69 and 73 for the seven
-  // launches of the many-block kernels.
-  const bool one = !deep && n <= bh_cluster_max();
+  // capacity, where the device has room for it: 20 us at 5k points and 28 at
+  // 10k against 69 and 73 for the seven launches of the many-block kernels.
+  const bool one = !deep && bh_cluster_fits(ctx, n);
   if (one) {
     timer_begin(ctx, FX_STAGE_BH_SORT, s, &ev);
     FX_TRY(bh_cluster_sort(ctx, x, y, n, b.bbox.p, th2, md2, b.keys[0].p, b.idx[0].p, b.spos.p,

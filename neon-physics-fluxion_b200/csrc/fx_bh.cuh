@@ -127,10 +127,11 @@ __device__ __forceinline__ unsigned match_digit(uint32_t d) {
 }
 
 // Keys, stable sort, sorted positions, root square and the exact sums of every
-// 512 consecutive points (tile_sum: ceil(n / 512) of them) of up to
-// bh_cluster_max() points in one launch (fx_bh_sort.cu); for positions whose
-// keys need no deep levels. Re-arms bbox.
-int bh_cluster_max();
+// 512 consecutive points (tile_sum: ceil(n / 512) of them) in one launch
+// (fx_bh_sort.cu), where bh_cluster_fits: up to 32,768 points, and a device
+// share with room for the cluster; for positions whose keys need no deep
+// levels. Re-arms bbox.
+bool bh_cluster_fits(fx_ctx *ctx, int n);
 int bh_cluster_sort(fx_ctx *ctx, const float *x, const float *y, int n, unsigned int *bbox,
                     float th2, float md2, uint32_t *keys, int32_t *idx, float2 *spos,
                     ulonglong4 *tile_sum, float *root, cudaStream_t s);

@@ -18,6 +18,8 @@
 // kernels have caught up.
 #include <cooperative_groups.h>
 
+#include <cstdlib>
+
 #include "fx_bh.cuh"
 #include "fx_internal.h"
 
@@ -205,6 +207,36 @@ bh_cluster_sort_kernel(const float *__restrict__ px, const float *__restrict__ p
   }
 }
 
+// Whether the device has room for one cluster of this size: a process limited
+// to a share of the SMs may not.
+template <int kItems>
+bool cluster_fits() {
+  constexpr int smem = (int)sizeof(ClSmem<kItems>);
+  if (raise_smem_limit((const void *)bh_cluster_sort_kernel<kItems>, smem) != FX_OK) return false;
+  cudaLaunchAttribute dim{};
+  dim.id = cudaLaunchAttributeClusterDimension;
+  dim.val.clusterDim.x = kCl;
+  dim.val.clusterDim.y = dim.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kCl);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = &dim;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, bh_cluster_sort_kernel<kItems>, &cfg) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return clusters > 0;
+}
+
+int items_for(int n) {
+  const int need = (n + kCl * kClThreads - 1) / (kCl * kClThreads);
+  return need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : 8;
+}
+
 template <int kItems>
 int launch_sort(const float *x, const float *y, int n, unsigned int *bbox, float th2, float md2,
                 uint32_t *keys, int32_t *idx, float2 *spos, ulonglong4 *tile_sum, float *root,
@@ -219,7 +251,22 @@ int launch_sort(const float *x, const float *y, int n, unsigned int *bbox, float
 
 }  // namespace
 
-int bh_cluster_max() { return kClMax; }
+// Asked once per context and size; never where the environment variable
+// FLUXION_BH_CLUSTER is 0 (a test setting).
+bool bh_cluster_fits(fx_ctx *ctx, int n) {
+  if (n <= 0 || n > kClMax) return false;
+  static const bool off = [] {
+    const char *e = std::getenv("FLUXION_BH_CLUSTER");
+    return e && std::atoi(e) == 0;
+  }();
+  if (off) return false;
+  const int items = items_for(n);
+  signed char &fits = ctx->sort_cluster_fits[items == 8 ? 3 : items / 2];
+  if (fits < 0)
+    fits = items == 1 ? cluster_fits<1>() : items == 2 ? cluster_fits<2>()
+           : items == 4 ? cluster_fits<4>() : cluster_fits<8>();
+  return fits > 0;
+}
 
 int bh_cluster_sort(fx_ctx *ctx, const float *x, const float *y, int n, unsigned int *bbox,
                     float th2, float md2, uint32_t *keys, int32_t *idx, float2 *spos,
@@ -229,9 +276,9 @@ int bh_cluster_sort(fx_ctx *ctx, const float *x, const float *y, int n, unsigned
     set_error("bh_cluster_sort: %d points exceed %d", n, kClMax);
     return FX_EINVAL;
   }
-  const int need = (n + kCl * kClThreads - 1) / (kCl * kClThreads);
-  const auto f = need <= 1 ? launch_sort<1> : need <= 2 ? launch_sort<2>
-                 : need <= 4 ? launch_sort<4> : launch_sort<8>;
+  const int items = items_for(n);
+  const auto f = items == 1 ? launch_sort<1> : items == 2 ? launch_sort<2>
+                 : items == 4 ? launch_sort<4> : launch_sort<8>;
   FX_TRY(f(x, y, n, bbox, th2, md2, keys, idx, spos, tile_sum, root, s));
   ctx->launches += 1;
   return FX_OK;

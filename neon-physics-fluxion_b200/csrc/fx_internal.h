@@ -281,6 +281,9 @@ struct fx_ctx {
   // sin(i * 2.71828), the power iteration's start vector: a table of the
   // largest cluster seen (fx_partition.cu)
   fx::DevBuf<float> sin_tab;
+  // whether the Barnes-Hut sort's cluster of 1, 2, 4, 8 points a thread fits
+  // this device share (-1: not asked yet)
+  signed char sort_cluster_fits[4] = {-1, -1, -1, -1};
   int leaf_schedule = 0;           // last autotuned leaf schedule
   // FX_LEAF_AUTO decisions by batch shape (leaf count, mean leaf size and
   // iteration count, each as a power-of-two bucket)
