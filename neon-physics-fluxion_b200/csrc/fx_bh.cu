@@ -1320,6 +1320,15 @@ static int batch_stack_cap() {
   return cap;
 }
 
+// Whether the batched walk's arithmetic stays finite: it adds a point's term to
+// itself as k / min_dist^3 times a zero difference, and lanes that take no part
+// in an entry as 0 / d^3, with a reciprocal root that is infinite for a
+// subnormal square. The group walk leaves both out, at any distance floor.
+static bool batch_finite(float k, float md2) {
+  const double inv = 1.0 / std::sqrt((double)md2);
+  return md2 >= FLT_MIN && std::fabs((double)k) * inv * inv * inv < 0.25 * FLT_MAX;
+}
+
 // Two entries side by side, one half of each packed register: -x and -y of
 // their centres (head and tail), k * mass, lane mask, size^2. 80 bytes, so
 // that the lanes' stores to their halves conflict two ways at most.
@@ -1399,7 +1408,8 @@ bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__re
     sp = 1;
   }
   __syncwarp();
-  bool overflow = false;
+  bool overflow = stack_cap == 0;  // no batched walk at all (batch_finite)
+  if (overflow) sp = 0;
   while (sp > 0) {
     // pop up to eight opened cells: lane l takes child l % 4 of cell l / 4
     const int cnt = min(sp, 8);
@@ -1476,7 +1486,7 @@ bh_batch_walk_kernel(int n, const float2 *__restrict__ spos, const int32_t *__re
     };
     // their terms; m: k * mass, 0 where a lane takes none
     auto pair_add = [&](uint64_t m, float2 r2c, uint64_t dx, uint64_t dy) {
-      // r2c >= md2 > 0: never subnormal
+      // r2c >= md2, which batch_finite keeps normal
       const uint64_t inv = pack2(rsqrt_approx_ftz(r2c.x), rsqrt_approx_ftz(r2c.y));
       const uint64_t f = mul2(mul2(mul2(m, inv), inv), inv);
       fx2 = fma2(f, dx, fx2);
@@ -1792,10 +1802,11 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
           n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err);
   } else {
     const int wb = (n + 31) / 32;
+    const int cap = batch_finite(k, md2) ? batch_stack_cap() : 0;
 #define FX_FAST_WALK(ST, CNT)                                                             \
   bh_batch_walk_kernel<ST, CNT><<<wb, 32, 0, s>>>(                                        \
       n, b.spos.p, b.idx[0].p, b.qchild.p, b.node.p, k, th2, md2, b.force.p, err, term_count, \
-      batch_stack_cap())
+      cap)
     if (deep) {
       if (term_count) FX_FAST_WALK(kStackDeep, true);
       else FX_FAST_WALK(kStackDeep, false);
