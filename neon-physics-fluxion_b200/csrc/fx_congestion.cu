@@ -112,9 +112,11 @@ cong_scan_rows_kernel(int32_t *__restrict__ diff, int cols, int rows) {
 // Column scan over stripes of W columns, 1024 / W runs of rows to a column:
 // produces the counts, zeroes the difference array for the next call, and
 // reduces the overflow max(0, h + v - capacity) (grid.rs:71-91) as an FP64 sum
-// and an f32 max. Narrow stripes spread the grid over the SMs and leave a
-// thread few rows, which it then keeps in registers between its two passes:
-// 7.8 us at 512 x 512 (ncu cold; 13.4 with stripes of 32 columns, 16 blocks).
+// and an f32 max. A thread whose run has at most kScanKeep rows keeps them in
+// registers between its two passes: 7.8 us at 512 x 512 in stripes of 8 (ncu
+// cold; 13.4 in stripes of 32, whose runs of 16 rows are read twice).
+constexpr int kScanKeep = 8;
+
 template <int W>
 __global__ void __launch_bounds__(1024)
 cong_scan_cols_kernel(int32_t *__restrict__ diff, uint32_t *__restrict__ counts,
@@ -122,7 +124,7 @@ cong_scan_cols_kernel(int32_t *__restrict__ diff, uint32_t *__restrict__ counts,
                       double *__restrict__ partial, float *__restrict__ pmax,
                       unsigned int *__restrict__ done, double *__restrict__ result,
                       float *__restrict__ result_max) {
-  constexpr int kRuns = 1024 / W, kKeep = 8, kPer = kRuns / 32;
+  constexpr int kRuns = 1024 / W, kKeep = kScanKeep, kPer = kRuns / 32;
   const int t = threadIdx.x, tx = t % W, ty = t / W;
   const int c = blockIdx.x * W + tx;
   const int ld = cols + 1;
@@ -220,17 +222,28 @@ cong_scan_cols_kernel(int32_t *__restrict__ diff, uint32_t *__restrict__ counts,
   }
 }
 
-// Blocks' partial results fit 4096 slots: stripes of 8 columns up to 32,768.
+// The widest stripe whose runs stay in registers, and stripes of 32 where none
+// does (whole 128-byte lines: rows are read twice there) or where the blocks'
+// partial results, 4096 slots, would not fit. The congestion stage of 200k
+// gates in us, stripes of 8, 16, 32: 256 x 256 40, 40, 39; 512 x 512 39, 39,
+// 45; 1024 x 1024 43, 71, 68; 2048 x 2048 295, 192, 143; 8192 columns of 256
+// rows 65, 55, 49; 4096 of 512 56, 51, 58.
+template <int W>
+static bool scan_kept(int cols, int rows) {
+  return rows <= 1024 / W * kScanKeep && cols <= 4096 * W;
+}
+
 static void launch_scan_cols(int32_t *diff, uint32_t *counts, int cols, int rows, float cap,
                              double *partial, float *pmax, unsigned int *done, double *result,
                              float *result_max, cudaStream_t s) {
-  if (cols <= 4096 * 8)
-    cong_scan_cols_kernel<8><<<(cols + 7) / 8, 1024, 0, s>>>(diff, counts, cols, rows, cap, partial,
-                                                             pmax, done, result, result_max);
-  else
-    cong_scan_cols_kernel<32><<<(cols + 31) / 32, 1024, 0, s>>>(diff, counts, cols, rows, cap,
-                                                                partial, pmax, done, result,
-                                                                result_max);
+  auto run = [&](auto kernel, int w) {
+    kernel<<<(cols + w - 1) / w, 1024, 0, s>>>(diff, counts, cols, rows, cap, partial, pmax, done,
+                                               result, result_max);
+  };
+  if (scan_kept<32>(cols, rows)) run(cong_scan_cols_kernel<32>, 32);
+  else if (scan_kept<16>(cols, rows)) run(cong_scan_cols_kernel<16>, 16);
+  else if (scan_kept<8>(cols, rows)) run(cong_scan_cols_kernel<8>, 8);
+  else run(cong_scan_cols_kernel<32>, 32);
 }
 
 int congestion_alloc(fx_design *d, int cols, int rows, cudaStream_t s) {
