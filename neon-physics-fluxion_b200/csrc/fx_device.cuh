@@ -138,11 +138,12 @@ __device__ __forceinline__ void agg_add_u64(unsigned long long *base, long long 
   if (i >= 0 && lane == (unsigned)(__ffs(peers) - 1)) red_add_global(base + i, sum);
 }
 
-// Adds the same constant `v` from every lane naming idx (>= 0).
-__device__ __forceinline__ void agg_add_const_i32(int *base, long long idx, int v) {
+// Adds the same constant `v` from every lane naming idx (>= 0); `few`: into so
+// few elements that lanes are likely to meet anyway, and are always matched.
+__device__ __forceinline__ void agg_add_const_i32(int *base, long long idx, int v, bool few) {
   const unsigned lane = threadIdx.x & 31u;
   const int i = (int)idx;  // indexes fit 31 bits
-  if (!crowded(i)) {
+  if (!few && !crowded(i)) {
     if (i >= 0) red_add_global(base + i, v);
     return;
   }

@@ -1,5 +1,6 @@
 """Congestion grids on both sides of each limit of the column scan's stripes (256, 512 and 1024 rows;
-columns past 4096 stripes of 8 and 16), against the oracle's counts. The counts are whole numbers; the
+columns past 4096 stripes of 8 and 16) and of the cells below which a warp's increments are always
+matched (4096), against the oracle's counts. The counts are whole numbers; the
 overflow is an FP64 sum of f32 terms, within cells x 2^-53 of the exact one in any order."""
 import math
 
@@ -9,7 +10,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cols,rows", [(1, 1), (33, 256), (33, 257), (100, 512), (100, 513),
+@pytest.mark.parametrize("cols,rows", [(1, 1), (8, 8), (63, 65), (64, 64), (33, 256), (33, 257), (100, 512), (100, 513),
                                        (70, 1024), (70, 1025), (5, 4097), (2050, 1031),
                                        (32768, 600), (32769, 600), (65537, 300), (131072, 3)])
 def test_counts_and_overflow(fx, ctx, oracle, cols, rows):
