@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -302,6 +303,10 @@ struct fx_design {
   double area_sum = 0.0;         // of all gates
   std::vector<int32_t> h_adj_ptr, h_adj_idx;
   std::vector<float> h_w, h_h;
+  // gate -> slot of a leaf on the host (fx_leaf.cu: batches that repeat a
+  // gate); all -1 between uses
+  std::vector<int32_t> h_slot;
+  std::mutex h_slot_mu;
   // state: ping-pong positions, velocities
   fx::DevBuf<float> x[2], y[2];
   int cur = 0;

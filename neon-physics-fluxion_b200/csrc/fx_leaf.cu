@@ -583,15 +583,25 @@ static std::vector<int32_t> leaf_order(int L, const int32_t *leaf_ptr) {
 // to 16 threads, this took most of a call (16 of 19 ms for 16,384 leaves,
 // whose kernel runs 3 ms).
 
-// map[g] = slot of gate g (-1 before); flag: 1 a gate out of range, 2 a gate
-// listed twice.
+// map[g] = last slot of gate g (-1 before); flag: 1 a gate out of range, 2 a
+// gate listed twice.
 __global__ void leaf_map_kernel(const int32_t *__restrict__ gate, int G, int n,
                                 int32_t *__restrict__ map, unsigned int *__restrict__ flag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= G) return;
   const int g = gate[i];
   if (g < 0 || g >= n) atomicOr(flag, 1u);
-  else if (atomicExch(map + g, i) != -1) atomicOr(flag, 2u);
+  else if (atomicMax(map + g, i) != -1) atomicOr(flag, 2u);
+}
+
+// The reference writes the positions slot by slot, leaf by leaf, so a gate
+// listed more than once keeps its last slot's position. The placing kernels
+// write concurrently: every slot but a gate's last becomes ~gate and skips the
+// write.
+__global__ void leaf_last_kernel(int32_t *__restrict__ gate, int G,
+                                 const int32_t *__restrict__ map) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < G && map[gate[i]] != i) gate[i] = ~gate[i];
 }
 
 // A warp per leaf: counts its gates' in-leaf neighbours, takes the leaf's
@@ -643,6 +653,31 @@ leaf_adj_kernel(int L, const int32_t *__restrict__ gptr, const int32_t *__restri
   }
 }
 
+// The design's gate -> slot map on the host, all -1 between uses, for whoever
+// holds h_slot_mu. It is kept: filling one took 80 us of a call at 200k gates.
+static std::vector<int32_t> &slot_map(fx_design *d) {
+  if (d->h_slot.empty()) d->h_slot.assign((size_t)d->n, -1);
+  return d->h_slot;
+}
+
+// leaf_map_kernel's flag, on the host: for batches of up to this many gates,
+// whose check (about 5 ns a gate) costs less than waiting for the device's.
+constexpr int kHostCheck = 8192;
+static unsigned int leaf_flag(fx_design *d, const int32_t *gate, int G) {
+  std::lock_guard<std::mutex> lock(d->h_slot_mu);
+  std::vector<int32_t> &slot = slot_map(d);
+  unsigned int flag = 0;
+  for (int i = 0; i < G; ++i) {
+    const int32_t g = gate[i];
+    if (g < 0 || g >= d->n) flag |= 1u;
+    else if (slot[g] != -1) flag |= 2u;
+    else slot[g] = i;
+  }
+  for (int i = 0; i < G; ++i)
+    if (gate[i] >= 0 && gate[i] < d->n) slot[gate[i]] = -1;
+  return flag;
+}
+
 // In-leaf adjacency on the host, for batches that list a gate more than once.
 struct LeafHost {
   std::vector<int32_t> aptr;
@@ -685,7 +720,7 @@ static void leaf_adjacency(const fx_design *d, int l0, int l1, const int32_t *le
   }
 }
 
-static int build_leaf_host(const fx_design *d, int L, const int32_t *leaf_ptr,
+static int build_leaf_host(fx_design *d, int L, const int32_t *leaf_ptr,
                            const int32_t *leaf_gate, LeafHost &h) {
   const int32_t G = leaf_ptr[L];
   for (int32_t i = 0; i < G; ++i)
@@ -700,8 +735,8 @@ static int build_leaf_host(const fx_design *d, int L, const int32_t *leaf_ptr,
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
   const int nt = G >= 65536 ? (int)std::min<unsigned>(std::min(hw, 16u), (unsigned)L) : 1;
   if (nt <= 1) {
-    std::vector<int32_t> local((size_t)d->n, -1);
-    leaf_adjacency(d, 0, L, leaf_ptr, leaf_gate, local, h.aptr.data(), h.aidx);
+    std::lock_guard<std::mutex> lock(d->h_slot_mu);
+    leaf_adjacency(d, 0, L, leaf_ptr, leaf_gate, slot_map(d), h.aptr.data(), h.aidx);
   } else {
     std::vector<int> cut(nt + 1, L);
     cut[0] = 0;
@@ -861,16 +896,20 @@ extern "C" int fx_hapr_place_leaves(fx_ctx *ctx, fx_design *d, int32_t n_leaves,
   FX_CHECK_CUDA(up(order.p, host_order.data(), host_order.size() * 4));
   FX_CHECK_CUDA(up(reg.p, region, (size_t)n_leaves * 16));
   // slots of the gates, and whether each is listed once and in range
-  unsigned int flag = 0;
+  unsigned int flag = G <= kHostCheck ? leaf_flag(d, leaf_gate, G) : 0;
   FX_CHECK_CUDA(cudaMemsetAsync(map.p, 0xff, (size_t)d->n * 4, s));
   FX_CHECK_CUDA(cudaMemsetAsync(counter.p, 0, 16, s));
   if (G > 0) {
     leaf_map_kernel<<<(G + 255) / 256, 256, 0, s>>>(gate.p, G, d->n, map.p, counter.p + 2);
     FX_CHECK_LAUNCH();
     ctx->launches += 1;
+  }
+  if (G > kHostCheck) {
     FX_CHECK_CUDA(cudaMemcpyAsync(&flag, counter.p + 2, 4, cudaMemcpyDeviceToHost, s));
     FX_CHECK_CUDA(cudaStreamSynchronize(s));
   }
+  LeafHost h;
+  std::vector<int2> host_rows;
   if (flag == 0) {
     FX_TRY(aidx.alloc(d->a > 0 ? (size_t)d->a : 1));
     leaf_adj_kernel<<<(n_leaves + 7) / 8, 256, 0, s>>>(n_leaves, gptr.p, gate.p, map.p,
@@ -879,26 +918,15 @@ extern "C" int fx_hapr_place_leaves(fx_ctx *ctx, fx_design *d, int32_t n_leaves,
     FX_CHECK_LAUNCH();
     ctx->launches += 1;
   } else {
-    LeafHost h;
     FX_TRY(build_leaf_host(d, n_leaves, leaf_ptr, leaf_gate, h));
-    // The reference writes the positions slot by slot, leaf by leaf, so a gate
-    // listed more than once keeps its last slot's position. The kernels write
-    // concurrently: every slot but a gate's last goes up as ~gate and skips
-    // the write.
-    std::vector<int32_t> gate_last(leaf_gate, leaf_gate + G);
-    std::vector<uint8_t> seen((size_t)d->n, 0);
-    for (int32_t i = G - 1; i >= 0; --i) {
-      const int32_t g = leaf_gate[i];
-      if (seen[g]) gate_last[i] = ~g;
-      seen[g] = 1;
-    }
+    leaf_last_kernel<<<(G + 255) / 256, 256, 0, s>>>(gate.p, G, map.p);
+    FX_CHECK_LAUNCH();
+    ctx->launches += 1;
     FX_TRY(aidx.alloc(h.aidx.empty() ? 1 : h.aidx.size()));
-    FX_CHECK_CUDA(up(gate.p, gate_last.data(), (size_t)G * 4));
-    std::vector<int2> host_rows((size_t)G);
+    host_rows.resize((size_t)G);
     for (int32_t i = 0; i < G; ++i) host_rows[i] = make_int2(h.aptr[i], h.aptr[(size_t)i + 1]);
     FX_CHECK_CUDA(up(rows.p, host_rows.data(), (size_t)G * 8));
     FX_CHECK_CUDA(up(aidx.p, h.aidx.data(), h.aidx.size() * 2));
-    FX_CHECK_CUDA(cudaStreamSynchronize(s));  // the host arrays go out of scope
   }
   // gates outside the batch keep the caller's positions
   if (flag != 0 || G != d->n) {
