@@ -228,12 +228,16 @@ cong_scan_cols_kernel(int32_t *__restrict__ diff, uint32_t *__restrict__ counts,
   }
 }
 
-// The widest stripe whose runs stay in registers, and stripes of 32 where none
-// does (whole 128-byte lines: rows are read twice there) or where the blocks'
-// partial results, 4096 slots, would not fit. The congestion stage of 200k
-// gates in us, stripes of 8, 16, 32: 256 x 256 40, 40, 39; 512 x 512 39, 39,
-// 45; 1024 x 1024 43, 71, 68; 2048 x 2048 295, 192, 143; 8192 columns of 256
-// rows 65, 55, 49; 4096 of 512 56, 51, 58.
+// Stripes of 8 while the blocks are one wave and their runs stay in registers
+// (a small grid's scan is latency: 64 x 64 is 7.3 us alone in stripes of 32 and
+// costs a run of 10k gates 0.3 %); on wider grids the widest whose runs stay
+// there; stripes of 32 where none does (whole 128-byte lines: rows are read
+// twice there) or where the blocks' partial results, 4096 slots, would not fit.
+// The congestion stage of 200k gates in us, stripes of 8, 16, 32: 256 x 256 40,
+// 40, 39; 512 x 512 39, 39, 45; 1024 x 1024 43, 71, 68; 2048 x 2048 295, 192,
+// 143; 8192 columns of 256 rows 65, 55, 49; 4096 of 512 56, 51, 58.
+constexpr int kScanWave = 148 * 8;  // columns
+
 template <int W>
 static bool scan_kept(int cols, int rows) {
   return rows <= 1024 / W * kScanKeep && cols <= 4096 * W;
@@ -246,7 +250,8 @@ static void launch_scan_cols(int32_t *diff, uint32_t *counts, int cols, int rows
     kernel<<<(cols + w - 1) / w, 1024, 0, s>>>(diff, counts, cols, rows, cap, partial, pmax, done,
                                                result, result_max);
   };
-  if (scan_kept<32>(cols, rows)) run(cong_scan_cols_kernel<32>, 32);
+  if (cols <= kScanWave && scan_kept<8>(cols, rows)) run(cong_scan_cols_kernel<8>, 8);
+  else if (scan_kept<32>(cols, rows)) run(cong_scan_cols_kernel<32>, 32);
   else if (scan_kept<16>(cols, rows)) run(cong_scan_cols_kernel<16>, 16);
   else if (scan_kept<8>(cols, rows)) run(cong_scan_cols_kernel<8>, 8);
   else run(cong_scan_cols_kernel<32>, 32);

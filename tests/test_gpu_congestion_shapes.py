@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("cols,rows", [(1, 1), (8, 8), (63, 65), (64, 64), (33, 256), (33, 257), (100, 512), (100, 513),
-                                       (70, 1024), (70, 1025), (5, 4097), (2050, 1031),
+                                       (70, 1024), (70, 1025), (1184, 256), (1185, 256), (1185, 512),
+                                       (1185, 1024), (1184, 1025), (5, 4097), (2050, 1031),
                                        (32768, 600), (32769, 600), (65537, 300), (131072, 3)])
 def test_counts_and_overflow(fx, ctx, oracle, cols, rows):
     rng = np.random.default_rng(cols + rows)
