@@ -75,7 +75,8 @@ int fx_ctx_synchronize(fx_ctx *ctx);
 
 /* Stage identifiers for fx_ctx_stage_times. */
 #define FX_STAGE_ATTRACT_INTEGRATE 0 /* rows A+E fused                        */
-#define FX_STAGE_BH_KEYS           1 /* row B: Morton keys                    */
+#define FX_STAGE_BH_KEYS           1 /* row B: Morton keys (in the sort's time */
+                                     /* where one launch does both)           */
 #define FX_STAGE_BH_SORT           2 /* row B: radix sort                     */
 #define FX_STAGE_BH_TREE           3 /* row B: radix tree + mass sums         */
 #define FX_STAGE_BH_WALK           4 /* row B: warp-cooperative walk          */
