@@ -604,6 +604,30 @@ __global__ void leaf_last_kernel(int32_t *__restrict__ gate, int G,
   if (i < G && map[gate[i]] != i) gate[i] = ~gate[i];
 }
 
+// A gate's row is walked by its lane up to this many neighbours, by the whole
+// warp beyond: a lane takes two trips to memory per neighbour (a gate on 100k
+// nets 9 ms, by the warp 0.6).
+constexpr int kLaneRow = 64;
+constexpr int kRowBatch = 8;  // trips of the warp in flight
+
+// Slots in [b, e) of the neighbours q0 .. q1 of one gate, by the warp: take(slot
+// or -1) for 32 consecutive neighbours at a time, in order.
+template <class F>
+__device__ __forceinline__ void warp_row(const int32_t *__restrict__ adj_idx,
+                                         const int32_t *__restrict__ map, int q0, int q1, int b,
+                                         int e, F take) {
+  const int lane = threadIdx.x & 31;
+  for (int q = q0 + lane; q - lane < q1; q += 32 * kRowBatch) {
+    int t[kRowBatch];
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) t[u] = q + 32 * u < q1 ? adj_idx[q + 32 * u] : -1;
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) t[u] = t[u] >= 0 ? map[t[u]] : -1;
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) take(t[u] >= b && t[u] < e ? t[u] : -1);
+  }
+}
+
 // A warp per leaf: counts its gates' in-leaf neighbours, takes the leaf's
 // share of aidx from *total (rows of a leaf are dense and in slot order; where
 // the leaf's share lies depends on timing, what it holds does not), writes them.
@@ -612,44 +636,67 @@ leaf_adj_kernel(int L, const int32_t *__restrict__ gptr, const int32_t *__restri
                 const int32_t *__restrict__ map, const int32_t *__restrict__ adj_ptr,
                 const int32_t *__restrict__ adj_idx, unsigned int *__restrict__ total,
                 int2 *__restrict__ rows, int16_t *__restrict__ aidx) {
+  const unsigned full = 0xffffffffu;
   const int l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (l >= L) return;
   const int b = gptr[l], e = gptr[l + 1];
   int sum = 0;
-  for (int i = b + lane; i < e; i += 32) {
-    const int g = gate[i], q1 = adj_ptr[g + 1];
+  for (int i0 = b; i0 < e; i0 += 32) {
+    const int i = i0 + lane;
+    const int g = i < e ? gate[i] : -1;
+    const int q0 = g >= 0 ? adj_ptr[g] : 0, q1 = g >= 0 ? adj_ptr[g + 1] : 0;
+    const bool wide = q1 - q0 > kLaneRow;
     int c = 0;
-    for (int q = adj_ptr[g]; q < q1; ++q) {
-      const int t = map[adj_idx[q]];
-      c += t >= b && t < e;
+    if (!wide)
+      for (int q = q0; q < q1; ++q) {
+        const int t = map[adj_idx[q]];
+        c += t >= b && t < e;
+      }
+    for (unsigned m = __ballot_sync(full, wide); m; m &= m - 1u) {
+      const int src = __ffs(m) - 1;
+      int n = 0;
+      warp_row(adj_idx, map, __shfl_sync(full, q0, src), __shfl_sync(full, q1, src), b, e,
+               [&](int t) { n += t >= 0; });
+      n = __reduce_add_sync(full, n);
+      if (lane == src) c = n;
     }
-    rows[i].y = c;
+    if (i < e) rows[i].y = c;
     sum += c;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  sum = __reduce_add_sync(full, sum);
   int base = 0;
   if (lane == 0) base = (int)atomicAdd(total, (unsigned int)sum);
-  base = __shfl_sync(0xffffffffu, base, 0);
+  base = __shfl_sync(full, base, 0);
   for (int i0 = b; i0 < e; i0 += 32) {
     const int i = i0 + lane;
     const int c = i < e ? rows[i].y : 0;
     int inc = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      const int u = __shfl_up_sync(full, inc, o);
       if (lane >= o) inc += u;
     }
-    if (i < e) {
-      int at = base + inc - c;
-      rows[i] = make_int2(at, at + c);
-      const int g = gate[i], q1 = adj_ptr[g + 1];
-      for (int q = adj_ptr[g]; q < q1; ++q) {
+    int at = base + inc - c;
+    const int g = i < e ? gate[i] : -1;
+    const int q0 = g >= 0 ? adj_ptr[g] : 0, q1 = g >= 0 ? adj_ptr[g + 1] : 0;
+    const bool wide = q1 - q0 > kLaneRow;
+    if (i < e) rows[i] = make_int2(at, at + c);
+    for (unsigned m = __ballot_sync(full, wide); m; m &= m - 1u) {
+      const int src = __ffs(m) - 1;
+      int to = __shfl_sync(full, at, src);
+      warp_row(adj_idx, map, __shfl_sync(full, q0, src), __shfl_sync(full, q1, src), b, e,
+               [&](int t) {
+                 const unsigned in = __ballot_sync(full, t >= 0);
+                 if (t >= 0) aidx[to + __popc(in & ((1u << lane) - 1u))] = (int16_t)(t - b);
+                 to += __popc(in);
+               });
+    }
+    if (!wide)
+      for (int q = q0; q < q1; ++q) {
         const int t = map[adj_idx[q]];
         if (t >= b && t < e) aidx[at++] = (int16_t)(t - b);
       }
-    }
-    base += __shfl_sync(0xffffffffu, inc, 31);
+    base += __shfl_sync(full, inc, 31);
   }
 }
 
