@@ -49,7 +49,7 @@ struct LeafBatch {
   const int16_t *aidx;     // in-leaf neighbour local indices (reference order)
   const float4 *region;    // [L] (cx, cy, w, h)
   const int32_t *order;    // [L] leaves in processing order
-  int n_leaves;
+  int n_leaves, gates;
   int iters;
   float k, repel, damping, dt;
   float *out_x, *out_y;    // global positions (written for leaf gates)
@@ -82,9 +82,9 @@ __device__ __forceinline__ float2 leaf_pair_force(float ax, float ay, float bx, 
 // operations of leaf_pair_force bit for bit: two partners to a packed f32x2
 // instruction (each half rounds as the scalar one; x - y as y * -1 + x), and
 // the reciprocal root without the subnormal handling its argument, >= 0.01,
-// never needs. Bound by the FP32 pipe and the reciprocal roots (eight cycles a
-// partner each): 2.98 to 2.52 ms for 16,384 leaves of 16-128 gates and 50
-// iterations (64 threads a leaf).
+// never needs. For batches that fill the device (launch_leaf). Bound by the
+// FP32 pipe and the reciprocal roots (eight cycles a partner each): 2.98 to 2.52
+// ms for 16,384 leaves of 16-128 gates and 50 iterations (64 threads a leaf).
 __device__ __forceinline__ void leaf_four_fast(uint64_t xi2, uint64_t yi2, const float *sx,
                                                const float *sy, uint64_t repel2, float *tx,
                                                float *ty) {
@@ -127,7 +127,7 @@ __device__ __forceinline__ void group_sync(int id) {
 
 // One leaf on a group of T threads (tid in [0, T)); sm: the group's shared
 // arrays x, y, vx, vy, fx, fy (kLeafMax each).
-template <int T, bool Fast>
+template <int T, bool Fast, bool Packed>
 __device__ void place_leaf(const LeafBatch &b, int leaf, int tid, float *sm, int sid) {
   float *sx = sm, *sy = sm + kLeafMax, *svx = sm + 2 * kLeafMax;
   float *svy = sm + 3 * kLeafMax, *sfx = sm + 4 * kLeafMax, *sfy = sm + 5 * kLeafMax;
@@ -163,17 +163,17 @@ __device__ void place_leaf(const LeafBatch &b, int leaf, int tid, float *sm, int
       const uint64_t xi2 = pack2(xi, xi), yi2 = pack2(yi, yi), rp2 = pack2(b.repel, b.repel);
       for (; m + kPairUnroll <= n; m += kPairUnroll) {
         float tx[kPairUnroll], ty[kPairUnroll];
-        if (Fast) {
+        if (Packed) {
           leaf_four_fast(xi2, yi2, sx + m, sy + m, rp2, tx, ty);
         } else {
 #pragma unroll
           for (int u = 0; u < kPairUnroll; ++u) {
-            const float2 t = leaf_pair_force<false>(xi, yi, sx[m + u], sy[m + u], b.repel);
+            const float2 t = leaf_pair_force<Fast>(xi, yi, sx[m + u], sy[m + u], b.repel);
             tx[u] = t.x;
             ty[u] = t.y;
           }
         }
-        if (Fast && (m ^ i) >= 32) {  // warp-uniform: none of these is a lane's own gate
+        if (Packed && (m ^ i) >= 32) {  // warp-uniform: none of these is a lane's own gate
 #pragma unroll
           for (int u = 0; u < kPairUnroll; ++u) {
             ax = __fadd_rn(ax, tx[u]);
@@ -220,7 +220,7 @@ __device__ void place_leaf(const LeafBatch &b, int leaf, int tid, float *sm, int
 }
 
 // T threads per leaf; the 256-thread block holds 256 / T groups.
-template <int T, bool Fast>
+template <int T, bool Fast, bool Packed>
 __global__ void __launch_bounds__(256)
 leaf_batch_kernel(LeafBatch b, int per_cluster_leaf) {
   extern __shared__ __align__(16) float lsm[];
@@ -229,7 +229,7 @@ leaf_batch_kernel(LeafBatch b, int per_cluster_leaf) {
   float *sm = lsm + grp * kLeafArrays * kLeafMax;
   const int sid = 1 + grp;
   if (per_cluster_leaf >= 0) {  // the one-launch-per-leaf baseline
-    if (grp == 0) place_leaf<T, Fast>(b, per_cluster_leaf, tid, sm, sid);
+    if (grp == 0) place_leaf<T, Fast, Packed>(b, per_cluster_leaf, tid, sm, sid);
     return;
   }
   __shared__ int next[kGroups];
@@ -242,7 +242,7 @@ leaf_batch_kernel(LeafBatch b, int per_cluster_leaf) {
     const int leaf = next[grp];
     group_sync<T>(sid);
     if (leaf < 0) break;
-    place_leaf<T, Fast>(b, leaf, tid, sm, sid);
+    place_leaf<T, Fast, Packed>(b, leaf, tid, sm, sid);
   }
 }
 
@@ -819,33 +819,63 @@ static int build_leaf_host(fx_design *d, int L, const int32_t *leaf_ptr,
   return FX_OK;
 }
 
-template <int T, bool Fast>
-static int launch_leaf(fx_ctx *ctx, const LeafBatch &b, bool per_cluster,
-                       cudaStream_t s) {
+// Blocks an SM of a per-gate schedule holds.
+template <int T, bool Fast, bool Packed>
+static int leaf_per_sm(int *per_sm) {
+  constexpr int smem = 256 / T * kLeafArrays * kLeafMax * (int)sizeof(float);
+  const auto kernel = leaf_batch_kernel<T, Fast, Packed>;
+  FX_TRY(raise_smem_limit(reinterpret_cast<const void *>(kernel), smem));
+  FX_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, 256, smem));
+  if (*per_sm < 1) *per_sm = 1;
+  return FX_OK;
+}
+
+template <int T, bool Fast, bool Packed>
+static int launch_leaf_as(fx_ctx *ctx, const LeafBatch &b, bool per_cluster, int sms,
+                          cudaStream_t s) {
   constexpr int kGroups = 256 / T;
   const size_t smem = (size_t)kGroups * kLeafArrays * kLeafMax * sizeof(float);
-  FX_TRY(raise_smem_limit(reinterpret_cast<const void *>(leaf_batch_kernel<T, Fast>),
-                          (int)smem));
+  int per_sm = 0;
+  FX_TRY((leaf_per_sm<T, Fast, Packed>(&per_sm)));
   if (per_cluster) {
     for (int l = 0; l < b.n_leaves; ++l)
-      leaf_batch_kernel<T, Fast><<<1, 256, smem, s>>>(b, l);
+      leaf_batch_kernel<T, Fast, Packed><<<1, 256, smem, s>>>(b, l);
     FX_CHECK_LAUNCH();
     ctx->launches += b.n_leaves;
     return FX_OK;
   }
-  int per_sm = 0;
-  FX_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, leaf_batch_kernel<T, Fast>, 256, smem));
-  if (per_sm < 1) per_sm = 1;
-  int grid = (ctx->persistent_sms > 0 ? ctx->persistent_sms : ctx->num_sms) * per_sm;
+  int grid = sms * per_sm;
   const int need = (b.n_leaves + kGroups - 1) / kGroups;
   if (grid > need) grid = need;
   if (grid < 1) grid = 1;
   FX_CHECK_CUDA(cudaMemsetAsync(b.counter, 0, 4, s));
-  leaf_batch_kernel<T, Fast><<<grid, 256, smem, s>>>(b, -1);
+  leaf_batch_kernel<T, Fast, Packed><<<grid, 256, smem, s>>>(b, -1);
   FX_CHECK_LAUNCH();
   ctx->launches += 1;
   return FX_OK;
+}
+
+// FX_LEAF_FAST by packed pairs where issue counts: two warps with gates or more
+// to a scheduler, and leaves that fill 5/16 of their threads. With fewer a
+// group's chain of terms is the time, and the scalar form's is the shorter.
+// Scalar and packed, us for 50 iterations: 64 leaves of 39 gates, 64 threads a
+// leaf 115 and 121; 300 of 100, 64 threads (one warp a scheduler) 361 and 410,
+// 128 threads (two) 283 and 260; 2,000 of 54, 64 threads 351 and 317, 256
+// threads (2 warps of 8 with gates) 399 and 447; 2,000 of 120, 256 threads 1063
+// and 915.
+template <int T, bool Fast>
+static int launch_leaf(fx_ctx *ctx, const LeafBatch &b, bool per_cluster, cudaStream_t s) {
+  const int sms = ctx->persistent_sms > 0 ? ctx->persistent_sms : ctx->num_sms;
+  if constexpr (Fast) {
+    int per_sm = 0;
+    FX_TRY((leaf_per_sm<T, true, true>(&per_sm)));
+    const int64_t resident = std::min<int64_t>(b.n_leaves, (int64_t)sms * per_sm * (256 / T));
+    const int mean = b.gates / std::max(1, b.n_leaves);
+    const int64_t warps = resident * ((std::min(mean, T) + 31) / 32);
+    if (!per_cluster && warps >= 8 * (int64_t)sms && 16 * mean >= 5 * T)
+      return launch_leaf_as<T, true, true>(ctx, b, per_cluster, sms, s);
+  }
+  return launch_leaf_as<T, Fast, false>(ctx, b, per_cluster, sms, s);
 }
 
 template <bool Fast>
@@ -985,7 +1015,7 @@ extern "C" int fx_hapr_place_leaves(fx_ctx *ctx, fx_design *d, int32_t n_leaves,
     FX_CHECK_CUDA(cudaMemsetAsync(d->leaf_trace.p, 0, (size_t)std::max(G, 1) * 8, s));
     d->leaf_trace_n = G;
   }
-  LeafBatch b{gptr.p, gate.p, rows.p, aidx.p, reg.p, order.p, n_leaves,
+  LeafBatch b{gptr.p, gate.p, rows.p, aidx.p, reg.p, order.p, n_leaves, G,
               cfg->force_iterations, cfg->attract_weight, cfg->repel_weight,
               cfg->damping, cfg->dt, ox.p, oy.p, counter.p,
               d->trace_on ? d->leaf_trace.p : nullptr};
