@@ -671,6 +671,22 @@ __host__ __device__ inline int pow2_above(int n) {
   while (p < n) p <<= 1;
   return p;
 }
+// In-cluster neighbours per cluster up to which that pays, with a fixed count
+// and with the stop rule. One block goes through them in each iteration (0.3 ns
+// a neighbour) where the kernels above spread them over the device. Whole calls,
+// ms, here against everything above: 2,500 gates of 21 neighbours 0.9 and 1.9,
+// of 51 1.7 and 1.1 (stop rule: 1.7 and 1.9), of 446 16 and 2.8 (16 and 6.4);
+// 4,096 of 3,509 180 and 16 (180 and 28).
+constexpr int64_t kSmallEdges = 1 << 16, kSmallEdgesStop = 1 << 18;
+
+// Rows so long that the one-launch form is the slower: a tile of its neighbours
+// holds few rows, each one lane's chain, and there are many tiles. 30,000 gates
+// of 6,993 neighbours 246 ms, stepped 90; of 1,172 28 and 29.
+constexpr int64_t kDenseEdges = 1 << 24;
+constexpr int kDenseRow = 512;
+static bool dense_rows(int64_t edges, int64_t positions) {
+  return edges > kDenseEdges && edges / std::max<int64_t>(positions, 1) > kDenseRow;
+}
 static size_t part_small_smem(int most) {
   return (size_t)pow2_above(most) * 8 + (size_t)most * 8 + ((size_t)most + 1) * 4;
 }
@@ -1051,6 +1067,7 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
     FX_TRY(rp.alloc((size_t)N + 1));
     FX_TRY(tsum.alloc((size_t)st + 1));
     FX_TRY(col.alloc(std::max<size_t>(d->adj_idx.n, 1)));
+    int64_t edges = d->a;  // in-cluster neighbours of the depth, at most
     for (int32_t depth = 0; depth < levels; ++depth) {
       // the clusters bisected at this depth, in position order (pre-order
       // lists them left to right within a depth)
@@ -1069,7 +1086,8 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       FX_TRY(upload(end, he, s));
       int32_t most = 0;
       for (int c = 0; c < C; ++c) most = std::max(most, he[c] - hb[c]);
-      if (!exact && most <= kPartChunk) {
+      const int64_t small_edges = cfg->tol > 0.0 ? kSmallEdgesStop : kSmallEdges;
+      if (!exact && most <= kPartChunk && edges / C <= small_edges) {
         // one block per cluster; two to four positions a thread
         const size_t smem = part_small_smem(most);
         const int threads = std::min(1024, std::max(96, (most / 2 + 31) / 32 * 32));
@@ -1133,7 +1151,8 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       const int grid = ctx->num_sms * (int)std::min<int64_t>(per_sm, (work + share - 1) / share);
       // positions of a block: its share, all positions without neighbours
       const int64_t per = grid > 0 ? ((int64_t)N + d->a / kPowerPos) / grid + 2 : N;
-      bool fixed = !exact && cfg->tol <= 0.0 && grid > 0 && per / least + 2 <= kPowerClusters;
+      bool fixed = !exact && cfg->tol <= 0.0 && grid > 0 && per / least + 2 <= kPowerClusters &&
+                   !dense_rows(edges, A);
       if (fixed) {
         FX_TRY(lv2.alloc(N));
         // the start vector is in v: x = v, and v gets the last one
@@ -1234,7 +1253,14 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       FX_CHECK_LAUNCH();
       ctx->launches += 3;
       cur ^= 1;
+      int32_t had = 0;
+      // the exact count where the next depth's choice may hang on it
+      const bool ask = !exact && ((most <= 2 * kPartChunk && edges / (2 * C) > small_edges) ||
+                                  dense_rows(edges, A));
+      if (ask)
+        FX_CHECK_CUDA(cudaMemcpyAsync(&had, rp.p + N, 4, cudaMemcpyDeviceToHost, s));
       FX_CHECK_CUDA(cudaStreamSynchronize(s));
+      if (ask) edges = had;
     }
     unsigned long long si = 0;
     unsigned int gave_up = 0;
