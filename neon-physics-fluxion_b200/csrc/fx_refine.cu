@@ -380,10 +380,11 @@ extern "C" int fx_refine(fx_ctx *ctx, fx_design *d, const fx_refine_cfg *cfg,
         cfg->move_distance, d->chip_w, d->chip_h, state.p);
     FX_CHECK_LAUNCH();
     ctx->launches += 2;
-    if (it > 0) {
-      FX_CHECK_CUDA(cudaEventSynchronize(done[(it - 1) & 1]));
-      stopped = seen(it - 1).stop != 0;
-    }
+    // (the first decision is waited for: a placement with nothing to refine is
+    // not counted a third time)
+    const int read = it > 0 ? it - 1 : 0;
+    FX_CHECK_CUDA(cudaEventSynchronize(done[read & 1]));
+    stopped = seen(read).stop != 0;
   }
   // the final count (the stopped loop's own, or that of the last moves)
   FX_TRY(congestion_run(ctx, d, px, py, cols, rows, s));
