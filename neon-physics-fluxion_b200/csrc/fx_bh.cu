@@ -1163,9 +1163,14 @@ bh_walk_kernel(int n, const float2 *__restrict__ spos,
 // schedulers idle. A cell's quad children are loaded with its record, so a
 // pass is one trip to memory. 10k points 69 us (group walk 174), 100k 247
 // (293), 130k 306 (332); at 300k, where issue counts, the group walk's 551
-// wins (729), hence the limit.
+// wins (729), hence the limit. At opening angle 0 every cell is opened and the
+// walk goes by all pairs, where issue counts much earlier: uniform points, 20k
+// 7.4 ms (group walk 11.6), 30k 14.9 (17.3), 40k 24.7 (23.4), 130k 209 (107). At
+// 0.02 the limit above still holds (130k 40, group walk 48).
 constexpr int kSmallWarps = 4;
 constexpr int kSmallWalkMax = 1 << 17;
+constexpr int kSmallWalkPairs = 1 << 15;  // below an angle of 0.001
+constexpr float kPairsTheta2 = 1e-6f;
 
 template <int Stack>
 __global__ void __launch_bounds__(kSmallWarps * 32)
@@ -1784,7 +1789,7 @@ int bh_run(fx_ctx *ctx, fx_design *d, float k, float theta, float min_dist, int 
   FX_CHECK_LAUNCH();
   timer_end(ctx, FX_STAGE_BH_TREE, s, ev);
   timer_begin(ctx, FX_STAGE_BH_WALK, s, &ev);
-  if (walk == FX_BH_EXACT && n <= kSmallWalkMax) {
+  if (walk == FX_BH_EXACT && n <= (th2 < kPairsTheta2 ? kSmallWalkPairs : kSmallWalkMax)) {
     const int wb = (n + kSmallWarps * 8 - 1) / (kSmallWarps * 8);
     if (deep)
       bh_small_walk_kernel<kStackDeep><<<wb, kSmallWarps * 32, 0, s>>>(
