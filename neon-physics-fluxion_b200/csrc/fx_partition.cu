@@ -684,8 +684,8 @@ constexpr int64_t kSmallEdges = 1 << 16, kSmallEdgesStop = 1 << 18;
 // of 6,993 neighbours 246 ms, stepped 90; of 1,172 28 and 29.
 constexpr int64_t kDenseEdges = 1 << 24;
 constexpr int kDenseRow = 512;
-static bool dense_rows(int64_t edges, int64_t positions) {
-  return edges > kDenseEdges && edges / std::max<int64_t>(positions, 1) > kDenseRow;
+static bool dense_rows(double per_gate, int64_t positions) {
+  return per_gate * (double)positions > kDenseEdges && per_gate > kDenseRow;
 }
 static size_t part_small_smem(int most) {
   return (size_t)pow2_above(most) * 8 + (size_t)most * 8 + ((size_t)most + 1) * 4;
@@ -1067,7 +1067,9 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
     FX_TRY(rp.alloc((size_t)N + 1));
     FX_TRY(tsum.alloc((size_t)st + 1));
     FX_TRY(col.alloc(std::max<size_t>(d->adj_idx.n, 1)));
-    int64_t edges = d->a;  // in-cluster neighbours of the depth, at most
+    // in-cluster neighbours a gate: the design's mean (a depth's is mostly
+    // lower), or the last depth's own where that was asked for
+    double per_gate = (double)d->a / (double)N;
     for (int32_t depth = 0; depth < levels; ++depth) {
       // the clusters bisected at this depth, in position order (pre-order
       // lists them left to right within a depth)
@@ -1087,7 +1089,9 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       int32_t most = 0;
       for (int c = 0; c < C; ++c) most = std::max(most, he[c] - hb[c]);
       const int64_t small_edges = cfg->tol > 0.0 ? kSmallEdgesStop : kSmallEdges;
-      if (!exact && most <= kPartChunk && edges / C <= small_edges) {
+      // of a cluster: by the mean, and at most all its pairs
+      auto cluster_edges = [&](double gates) { return std::min(gates, per_gate) * gates; };
+      if (!exact && most <= kPartChunk && cluster_edges(most) <= (double)small_edges) {
         // one block per cluster; two to four positions a thread
         const size_t smem = part_small_smem(most);
         const int threads = std::min(1024, std::max(96, (most / 2 + 31) / 32 * 32));
@@ -1152,7 +1156,7 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       // positions of a block: its share, all positions without neighbours
       const int64_t per = grid > 0 ? ((int64_t)N + d->a / kPowerPos) / grid + 2 : N;
       bool fixed = !exact && cfg->tol <= 0.0 && grid > 0 && per / least + 2 <= kPowerClusters &&
-                   !dense_rows(edges, A);
+                   !dense_rows(per_gate, A);
       if (fixed) {
         FX_TRY(lv2.alloc(N));
         // the start vector is in v: x = v, and v gets the last one
@@ -1255,12 +1259,13 @@ extern "C" int fx_partition(fx_ctx *ctx, fx_design *d, const fx_part_cfg *cfg,
       cur ^= 1;
       int32_t had = 0;
       // the exact count where the next depth's choice may hang on it
-      const bool ask = !exact && ((most <= 2 * kPartChunk && edges / (2 * C) > small_edges) ||
-                                  dense_rows(edges, A));
+      const bool ask =
+          !exact && ((most <= 2 * kPartChunk && cluster_edges(0.5 * most) > (double)small_edges) ||
+                     dense_rows(per_gate, A));
       if (ask)
         FX_CHECK_CUDA(cudaMemcpyAsync(&had, rp.p + N, 4, cudaMemcpyDeviceToHost, s));
       FX_CHECK_CUDA(cudaStreamSynchronize(s));
-      if (ask) edges = had;
+      if (ask) per_gate = (double)had / (double)A;
     }
     unsigned long long si = 0;
     unsigned int gave_up = 0;

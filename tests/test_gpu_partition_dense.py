@@ -64,3 +64,17 @@ def test_matches_restatement(fx, ctx, n, pins, nets, iters, tol, leaf):
         return build(o[:cut]) + build(o[cut:])
 
     assert np.array_equal(got["leaf_gate"], np.array(build(np.arange(n))))
+
+
+@pytest.mark.parametrize("tol", [0.0, 1e-6])
+def test_last_depth_of_few_clusters(fx, ctx, tol):
+    """51,201 gates in leaves of 50 have one depth more than 51,200, of a single cluster of 51 gates:
+    one launch, however many neighbours the whole design has."""
+    launches = []
+    for n in (51200, 51201):
+        d = fx.Design(ctx, fx.synth_plain(5, n, int(1.2 * n), float(1.2 * np.sqrt(n))).circuit)
+        at = ctx.kernel_launches()
+        d.partition(fx.part_cfg(mode=fx.FX_PART_FP64, power_iterations=3, tol=tol, max_leaf_size=50))
+        launches.append(ctx.kernel_launches() - at)
+        d.close()
+    assert launches[1] == launches[0] + 1, launches
